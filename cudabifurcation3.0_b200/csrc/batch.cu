@@ -52,14 +52,14 @@ __device__ __forceinline__ void bif_tile(const DevJob& J, void* out, int* aux, l
     if (TASK == CBF_TASK_PEAKS) {
         if (valid) {
             double* pk = (double*)out + p * (long long)J.peakCap;
-            aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, J.peakCap, nullptr, nullptr);
+            aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, J.peakCap, nullptr, nullptr, ring_column(L, lane));
         }
         return;
     }
     double* myPk = slotPk + (long long)lane * stride;
     double* myIv = (TASK == CBF_TASK_DBSCAN) ? slotIv + (long long)lane * stride : nullptr;
     int n = 0;
-    if (valid) n = integrate_point<S, TASK>(J, g, myPk, myIv, J.peakCap, nullptr, nullptr);
+    if (valid) n = integrate_point<S, TASK>(J, g, myPk, myIv, J.peakCap, nullptr, nullptr, ring_column(L, lane));
     __syncwarp();
     int res = 0;
     const int live = (int)min((long long)kTile, J.nPoints - p0);
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kBatchThreads, 6) batch_kernel(
     const BatchJob* __restrict__ jobs, int nJobs, const long long* __restrict__ tileEnd,
     unsigned long long* counter, double* scrPk, double* scrIv, int stride, int bitWords, int sortCap, int* err)
 {
-    extern __shared__ unsigned smem[];
+    extern __shared__ __align__(16) unsigned smem[];
     __shared__ long long sEnd[kMaxBatchJobs];
     for (int i = threadIdx.x; i < nJobs; i += blockDim.x) sEnd[i] = tileEnd[i];
     __syncthreads();

@@ -52,15 +52,23 @@ struct Overflow {
 };
 
 // ---------------------------------------------------------------------------
+// Blocks per SM the kernel is compiled for.  A lane has one chain of FP64 steps,
+// and a scheduler issues those best from a multiple of four warps: a bare chain
+// of the 8-instruction step reaches 0.71 of the FP64 pipe with 4 or 8 warps per
+// scheduler, 0.53 with 5 and 0.59 with 6 (the DBSCAN kernel's transient at 7 and
+// at 8 blocks: 72 and 64 ms for 1024^2 x 100 000 steps).
+template <class S>
+constexpr int kBifMinBlocks = S::DIM == 3 ? 8 : 4;
+
 template <class S, int TASK>
-__global__ void __launch_bounds__(kBifThreads) bif_kernel(const DevJob J, void* __restrict__ d_out,
+__global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(const DevJob J, void* __restrict__ d_out,
                                                           int* __restrict__ d_aux,
                                                           double* scrPeaks,
                                                           double* scrInt,
                                                           int bitWords, int sortCap,
                                                           int* __restrict__ err, const Overflow ov)
 {
-    extern __shared__ unsigned smem[];
+    extern __shared__ __align__(16) unsigned smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const long long warpId = (long long)blockIdx.x * kBifWarps + wib;
@@ -70,6 +78,7 @@ __global__ void __launch_bounds__(kBifThreads) bif_kernel(const DevJob J, void* 
     unsigned* L = smem + (size_t)wib * dbscan_warp_words(bitWords, sortCap);
     unsigned* Sb = L + bitWords;
     const DbscanSort so = dbscan_sort_area(L, bitWords, sortCap);
+    double* ring = ring_column(L, lane);
 
     for (long long tile = warpId; tile < nTiles; tile += nWarps) {
         const long long p = tile * 32 + lane;
@@ -79,14 +88,14 @@ __global__ void __launch_bounds__(kBifThreads) bif_kernel(const DevJob J, void* 
         if (TASK == CBF_TASK_PEAKS) {
             if (valid) {
                 double* pk = (double*)d_out + p * (long long)cap;
-                d_aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, cap, nullptr, nullptr);
+                d_aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, cap, nullptr, nullptr, ring);
             }
             continue;
         }
         if (TASK == CBF_TASK_TRAJECTORY) {
             if (valid) {
                 double* tr = (double*)d_out + p * (long long)cap;
-                integrate_point<S, TASK>(J, g, nullptr, nullptr, 0, tr, d_aux + p);
+                integrate_point<S, TASK>(J, g, nullptr, nullptr, 0, tr, d_aux + p, nullptr);
             }
             continue;
         }
@@ -97,7 +106,7 @@ __global__ void __launch_bounds__(kBifThreads) bif_kernel(const DevJob J, void* 
         int n = 0, div = 0;
         OstrovskyFlags of;
         of.init(J.ostThr);
-        if (valid) n = integrate_point<S, TASK>(J, g, myPk, myIv, cap, nullptr, &div, &of);
+        if (valid) n = integrate_point<S, TASK>(J, g, myPk, myIv, cap, nullptr, &div, ring, &of);
         // A truncated peak list whose result needs every peak goes to the second pass.
         const bool over = valid && ov.count && n > cap && n <= J.maxPeaks;
         if (over) {

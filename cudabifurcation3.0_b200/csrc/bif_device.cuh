@@ -3,53 +3,15 @@
 // epilogues.  Shared by the map kernel (bif.cu) and the batch kernel (batch.cu).
 #pragma once
 
+#include <type_traits>
+
 #include "engine.cuh"
+#include "peak_stream.cuh"
 
 namespace cbf {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-
-// ---------------------------------------------------------------------------
-// Streaming restatement of peakFinder (cudaLibrary.cu:220-266) over the samples
-// d[0..N) in arrival order.  Candidate i is judged when d[i+1] arrives:
-//   NORMAL : d[i] > d[i-1] && d[i] >= d[i+1] -> peak at i if d[i] > d[i+1],
-//            otherwise a plateau begins (inner loop of :229-246);
-//   PLATEAU: compare the plateau value with the next sample: larger -> peak at
-//            the plateau end j; smaller -> no peak; equal -> continue;
-//   SKIP   : after a peak or a rising plateau the reference sets i = j+1 and its
-//            ++i moves on to j+2, so the next arrival is not a candidate.
-// The first detected peak is dropped and intervals are (t[k+1]-t[k]) * 0.01
-// (:250-262).  NaN is absorbing for these systems, so the inner loop's
-// run-to-the-end case never yields a peak, as here.
-struct NoPeakHook {
-    __device__ __forceinline__ void operator()(double, int) const {}
-};
-
-// Flags of peakFinderCUDAForCalculationOfPeriodicityByOstrovsky
-// (cudaLibrary.cu:288-352) kept while the peaks stream by, over every peak:
-// non-increasing consecutive peaks (flag 0), peaks from the second on above /
-// not above the threshold (flags 1, 2), and the last recorded sample (flag 4).
-struct OstrovskyFlags {
-    double prev, last, thr;
-    bool nonInc, one, zero;
-    __device__ __forceinline__ void init(double threshold)
-    {
-        thr = threshold;
-        prev = last = 0.0;
-        nonInc = true;
-        one = zero = false;
-    }
-    __device__ __forceinline__ void operator()(double val, int k)
-    {
-        if (k >= 1) {
-            if (val - prev > 0) nonInc = false;
-            if (val > thr) one = true;
-            else zero = true;
-        }
-        prev = val;
-    }
-};
 
 // dbscanCUDAForCalculationOfPeriodicityByOstrovsky (cudaLibrary.cu:628-662):
 // the cluster count (dbscanDouble = dbscan as a double) rewritten by the flags.
@@ -82,73 +44,6 @@ __host__ __device__ constexpr bool task_with_intervals(int task)
     return task == CBF_TASK_DBSCAN || task == CBF_TASK_OSTROVSKY;
 }
 
-struct PeakStream {
-    double prev1, prev2, pval;
-    int mode;       // 0 NORMAL, 1 PLATEAU, 2 SKIP
-    int detected;
-    int lastT;
-
-    __device__ __forceinline__ void init()
-    {
-        prev1 = prev2 = pval = 0.0;
-        mode = 0;
-        detected = 0;
-        lastT = 0;
-    }
-
-    // hook(value, k) sees every emitted peak k = 0, 1, ... (also past cap).
-    template <bool WITH_INTERVALS, class Hook>
-    __device__ __forceinline__ void emit(double val, int t, double* pk, double* iv, int cap, Hook& hook)
-    {
-        if (detected >= 1) {
-            const int k = detected - 1;
-            hook(val, k);
-            if (k < cap) {
-                pk[k] = val;
-                if (WITH_INTERVALS) iv[k] = (double)(t - lastT) * kPeakIntervalUnit;
-            }
-        }
-        lastT = t;
-        ++detected;
-    }
-
-    template <bool WITH_INTERVALS>
-    __device__ __forceinline__ void push(double v, int t, double* pk, double* iv, int cap)
-    {
-        NoPeakHook h;
-        push<WITH_INTERVALS>(v, t, pk, iv, cap, h);
-    }
-
-    template <bool WITH_INTERVALS, class Hook>
-    __device__ __forceinline__ void push(double v, int t, double* pk, double* iv, int cap, Hook& hook)
-    {
-        if (t >= 2) {
-            if (mode == 2) {
-                mode = 0;
-            } else if (mode == 1) {
-                if (pval < v) {
-                    mode = 2;
-                } else if (pval > v) {
-                    emit<WITH_INTERVALS>(pval, t - 1, pk, iv, cap, hook);
-                    mode = 2;
-                }
-            } else if (prev1 > prev2 && prev1 >= v) {
-                if (prev1 > v) {
-                    emit<WITH_INTERVALS>(prev1, t - 1, pk, iv, cap, hook);
-                    mode = 2;
-                } else {
-                    mode = 1;
-                    pval = prev1;
-                }
-            }
-        }
-        prev2 = prev1;
-        prev1 = v;
-    }
-
-    __device__ __forceinline__ int emitted() const { return detected > 1 ? detected - 1 : 0; }
-};
-
 template <int D>
 __device__ __forceinline__ double pick(const double (&x)[D], int wv)
 {
@@ -159,53 +54,183 @@ __device__ __forceinline__ double pick(const double (&x)[D], int wv)
     return r;
 }
 
-// One point: transient (unchecked, cudaLibrary.cu:107-108), then the recorded
-// loop (:110-114) feeding the peak stream.  Returns the emitted peak count, 0 on
-// divergence (peakFinderCUDA turns the -1 flag into 0, :277-281).
-template <class S, int TASK>
-__device__ int integrate_point(const DevJob& J, long long g, double* pk, double* iv, int cap,
-                               double* traj, int* divFlag, OstrovskyFlags* of = nullptr)
+// The recorded variable of a state, physical; WV >= 0 fixes it at compile time.
+template <class S, int WV>
+__device__ __forceinline__ double sample_of(const double (&x)[S::DIM], int wv, const typename S::Coef& c)
+{
+    if constexpr (WV >= 0) return phys_comp<S>(x[WV], WV, c);
+    else return phys_comp<S>(pick<S::DIM>(x, wv), wv, c);
+}
+
+// Samples per block of the recorded loop, and the shared memory of a warp for
+// one block: rows 0..kRing of 32 doubles (row 0: the sample before the block).
+constexpr int kRing = 16;
+constexpr int kRingWords = (kRing + 1) * 32 * 2;
+
+// What the recorded loop needs of a job.
+struct RecordSpec {
+    int n, extra;     // samples; steps per sample - 1
+    int wv;
+    int checkDiv;
+    unsigned hiT;     // high word a sample must stay below in a block
+    int cap;          // peak slots of pk (and iv)
+    double divThresh;
+};
+
+template <class S>
+struct StateOf {
+    double x[S::DIM];
+};
+
+// The recorded loop (cudaLibrary.cu:110-114) feeding the peak stream; sample 0
+// is the state on entry.  Returns true if the divergence test fired.
+//
+// Bound: the FP64 step's operand reads.  Judging every sample as it arrives (two
+// FP64 comparisons, the divergence test, the state machine's branches) cost more
+// than the step: 103 ms for 40 000 samples x 1024^2 Lorenz points where 100 000
+// bare steps take 72 ms.  So samples are taken in blocks of kRing: per sample one
+// FP64 subtraction whose sign bit (d[i] above d[i-1]) is shifted into a mask, one
+// shared-memory store and half a three-input maximum against the threshold; the
+// block's peaks then follow from the mask's few candidates (44 ms; the 1024^2
+// DBSCAN map 256 -> 205 ms, a ragged batch 112 -> 86 ms).  A block in which a
+// sample may have reached the divergence threshold or is no number is repeated
+// from its first state with the exact per-sample code; so is the end of the
+// record.
+template <class S, int WV, bool PRE1, bool WITH_INTERVALS, class Hook>
+__device__ __forceinline__ bool record_loop(const RecordSpec& R, double (&x)[S::DIM], const typename S::Coef& c,
+                                            PeakStream& ps, double* ring, double* pk, double* iv, Hook& hook)
 {
     constexpr int D = S::DIM;
-    double x[D], v[CBF_MAX_VALUES];
-    setup_point<D>(J, g, x, v);
-    const typename S::Coef c = S::prep(v, J.h);
-    to_stored<S>(x, c);
-
-#pragma unroll 4
-    for (int i = 0; i < J.nSkip; ++i) S::step(x, c);
-
-    const int wv = J.writableVar;
-    PeakStream ps;
-    ps.init();
-    bool div = false;
-    int t = 0;
-    for (; t < J.nRecord; ++t) {
-        const double val = phys_comp<S>(pick<D>(x, wv), wv, c);
-        if (TASK == CBF_TASK_TRAJECTORY) {
-            traj[t] = val;
-        } else if (TASK == CBF_TASK_OSTROVSKY) {
-            of->last = val;
-            ps.push<true>(val, t, pk, iv, cap, *of);
-        } else {
-            ps.push<task_with_intervals(TASK)>(val, t, pk, iv, cap);
-        }
-        for (int j = 0; j < J.preScaller - 1; ++j) S::step(x, c);
+    const int n = R.n;
+    auto next = [&]() {
+        if (!PRE1)
+            for (int j = 0; j < R.extra; ++j) S::step(x, c);
         S::step(x, c);
-        if (J.checkDiv && diverged(phys_comp<S>(pick<D>(x, wv), wv, c), J.divThresh)) {
-            div = true;
-            ++t;
-            break;
+        return sample_of<S, WV>(x, R.wv, c);
+    };
+    if (n <= 0) return false;
+    int t = 0;  // the last sample fed
+    ps.push<WITH_INTERVALS>(sample_of<S, WV>(x, R.wv, c), 0, pk, iv, R.cap, hook);
+    while (t < n) {  // step t leads to sample t+1; the last one is only tested
+        int m = n - t;
+        if (m > kRing) {
+            double x0[D];
+#pragma unroll
+            for (int i = 0; i < D; ++i) x0[i] = x[i];
+            HiTrack tr;
+            tr.init();
+            unsigned up = 0;
+            double p = ps.prev1;
+            ring[0] = p;
+#pragma unroll 2
+            for (int i = 0; i < kRing; i += 2) {
+                const double a = next();
+                up = __funnelshift_l((unsigned)__double2hiint(p - a), up, 1);
+                ring[32 * i + 32] = a;
+                p = next();
+                up = __funnelshift_l((unsigned)__double2hiint(a - p), up, 1);
+                ring[32 * i + 64] = p;
+                tr.add2(a, p);
+            }
+            if (!tr.maybe(R.hiT)) {
+                ps.push_block<kRing, WITH_INTERVALS>(up, t, p, ring, pk, iv, R.cap, hook);
+                t += kRing;
+                continue;
+            }
+#pragma unroll
+            for (int i = 0; i < D; ++i) x[i] = x0[i];
+            m = kRing;
+        }
+        for (int i = 0; i < m; ++i) {
+            const double v = next();
+            if (R.checkDiv && diverged(v, R.divThresh)) return true;
+            if (++t < n) ps.push<WITH_INTERVALS>(v, t, pk, iv, R.cap, hook);
+            if (isnan(v)) return false;  // absorbing: no later sample is a peak or passes the test
         }
     }
-    if (TASK == CBF_TASK_OSTROVSKY) *divFlag = div ? 1 : 0;
-    if (TASK == CBF_TASK_TRAJECTORY) {
+    return false;
+}
+
+// The recorded loop of one point from state `st`: the emitted peak count, -1 if
+// the divergence test fired.  A function of its own, called once per point: its
+// registers are not those of the epilogues around it, and one copy serves all
+// tasks of a kernel.
+template <class S, bool WITH_INTERVALS, class Hook>
+__device__ __noinline__ int record_point(const RecordSpec R, StateOf<S> st, const typename S::Coef c, double* ring,
+                                         double* pk, double* iv, Hook* hookIO)
+{
+    Hook hook = *hookIO;
+    PeakStream ps;
+    ps.init();
+    bool div;
+    auto go = [&](auto wv) {
+        constexpr int WV = decltype(wv)::value;
+        return R.extra == 0 ? record_loop<S, WV, true, WITH_INTERVALS>(R, st.x, c, ps, ring, pk, iv, hook)
+                            : record_loop<S, WV, false, WITH_INTERVALS>(R, st.x, c, ps, ring, pk, iv, hook);
+    };
+    if constexpr (S::DIM == 3) {
+        if (R.wv == 0) div = go(std::integral_constant<int, 0>());
+        else if (R.wv == 1) div = go(std::integral_constant<int, 1>());
+        else div = go(std::integral_constant<int, 2>());
+    } else {
+        div = go(std::integral_constant<int, -1>());
+    }
+    if (R.n > 0) hook.finish(ps.prev1);
+    *hookIO = hook;
+    return div ? -1 : ps.emitted();
+}
+
+// One point: transient (unchecked, cudaLibrary.cu:107-108), then the recorded
+// loop (:110-114) feeding the peak stream.  Returns the emitted peak count, 0 on
+// divergence (peakFinderCUDA turns the -1 flag into 0, :277-281).  `ring`: this
+// lane's column of the warp's kRingWords (not used by TRAJECTORY).
+template <class S, int TASK>
+__device__ int integrate_point(const DevJob& J, long long g, double* pk, double* iv, int cap,
+                               double* traj, int* divFlag, double* ring, OstrovskyFlags* of = nullptr)
+{
+    constexpr int D = S::DIM;
+    StateOf<S> st;
+    typename S::Coef c;
+    {
+        double v[CBF_MAX_VALUES];
+        setup_point<D>(J, g, st.x, v);
+        c = S::prep(v, J.h);
+        to_stored<S>(st.x, c);
+    }
+
+#pragma unroll 4
+    for (int i = 0; i < J.nSkip; ++i) S::step(st.x, c);
+
+    if constexpr (TASK == CBF_TASK_TRAJECTORY) {
+        const int wv = J.writableVar;
+        bool div = false;
+        int t = 0;
+        for (; t < J.nRecord; ++t) {
+            traj[t] = phys_comp<S>(pick<D>(st.x, wv), wv, c);
+            for (int j = 0; j < J.preScaller; ++j) S::step(st.x, c);
+            if (J.checkDiv && diverged(phys_comp<S>(pick<D>(st.x, wv), wv, c), J.divThresh)) {
+                div = true;
+                ++t;
+                break;
+            }
+        }
         // Samples after a divergence are never written by the reference; make them NaN.
         for (; t < J.nRecord; ++t) traj[t] = __longlong_as_double(0x7ff8000000000000ll);
         *divFlag = div ? 1 : 0;
         return 0;
+    } else {
+        const RecordSpec R{J.nRecord, J.preScaller - 1, J.writableVar, J.checkDiv,
+                           J.checkDiv ? J.divHi : 0x7f800000u, cap, J.divThresh};
+        int n;
+        if constexpr (TASK == CBF_TASK_OSTROVSKY) {
+            n = record_point<S, true, OstrovskyFlags>(R, st, c, ring, pk, iv, of);
+            *divFlag = n < 0 ? 1 : 0;
+        } else {
+            NoPeakHook hook;
+            n = record_point<S, task_with_intervals(TASK), NoPeakHook>(R, st, c, ring, pk, iv, &hook);
+        }
+        return n < 0 ? 0 : n;
     }
-    return div ? 0 : ps.emitted();
 }
 
 // ---------------------------------------------------------------------------
@@ -322,10 +347,18 @@ struct DbscanSort {
 
 // 32-bit words of shared memory per warp: the bitsets L and S of `bitWords`
 // words each, and with `sortCap` > 0 (a power of two, 32..1024) also E, D and
-// the sort keys.
+// the sort keys.  The recorded loop's ring lies in the same words (a warp's
+// epilogues start when all its lanes have integrated).
 __host__ __device__ inline int dbscan_warp_words(int bitWords, int sortCap)
 {
-    return sortCap > 0 ? 4 * bitWords + sortCap : 2 * bitWords;
+    const int w = sortCap > 0 ? 4 * bitWords + sortCap : 2 * bitWords;
+    return w > kRingWords ? w : kRingWords;
+}
+
+// This lane's column of the ring that starts at the warp's shared words.
+__device__ __forceinline__ double* ring_column(unsigned* warpWords, int lane)
+{
+    return reinterpret_cast<double*>(warpWords) + lane;
 }
 
 // Sort keys per warp for peak lists of up to `peakCap` peaks: a power of two

@@ -10,8 +10,6 @@
 
 namespace cbf {
 
-constexpr double kPeakIntervalUnit = 0.01;  // peakFinder's default h (cudaLibrary.cuh:204)
-
 // A validated job in the form the kernels consume (passed by value).
 struct DevJob {
     double ranges[4];
@@ -117,36 +115,27 @@ __device__ __forceinline__ unsigned abs_hi(double v)
 
 // Conservative magnitude tracker of a stream of doubles against a threshold T:
 // |v| >= T needs hi(|v|) >= hi(T) (the high word is monotone in the magnitude),
-// and the signed high word of v is hi(|v|) for v >= 0, while its unsigned high
-// word is 2^31 + hi(|v|) for v < 0.  So the signed maximum of the high words
-// reaches hi(T) only if some positive value may have reached T, and the
-// unsigned maximum reaches 2^31 + hi(T) only if some negative one may have
-// (NaNs count as reaching it).  Two three-input maxima (the sm_90+ DPX integer
-// instructions) take two values per update with no masking: half the integer
-// work of tracking max |hi| of each value, which competes with the FP64 step
-// for issue slots.
+// and the high words compare like the floats of the same bits.  So one
+// three-input FP32 maximum of magnitudes (max.abs, sm_100) takes two values of
+// either sign per instruction; .NaN makes a high word that is no float number
+// (|v| >= 2^1017, infinities, NaNs) stick.  One instruction per two values
+// matters: what it reads from the register file delays the FP64 step, which is
+// bound by its own operand reads (a chain of the 8-instruction step with a
+// signed and an unsigned integer maximum per two values ran at 0.68 of the FP64
+// pipe, without any at 0.72).
 struct HiTrack {
-    int s;
-    unsigned u;
-    __device__ __forceinline__ void init()
-    {
-        s = INT_MIN;
-        u = 0;
-    }
+    float m;
+    __device__ __forceinline__ void init() { m = 0.0f; }
     __device__ __forceinline__ void add2(double a, double b)
     {
-        const int ha = __double2hiint(a), hb = __double2hiint(b);
-        s = __vimax3_s32(s, ha, hb);
-        u = __vimax3_u32(u, (unsigned)ha, (unsigned)hb);
+        asm("max.NaN.abs.f32 %0, %1, %2, %3;"
+            : "=f"(m)
+            : "f"(m), "f"(__int_as_float(__double2hiint(a))), "f"(__int_as_float(__double2hiint(b))));
     }
-    __device__ __forceinline__ void add1(double a)
-    {
-        const int ha = __double2hiint(a);
-        s = max(s, ha);
-        u = max(u, (unsigned)ha);
-    }
-    // hiT = the threshold's high word without sign (DevJob::divHi)
-    __device__ __forceinline__ bool maybe(unsigned hiT) const { return s >= (int)hiT || u >= 0x80000000u + hiT; }
+    __device__ __forceinline__ void add1(double a) { add2(a, a); }
+    // hiT = the threshold's high word without sign (DevJob::divHi); a NaN on
+    // either side reads as reached.
+    __device__ __forceinline__ bool maybe(unsigned hiT) const { return !(m < __uint_as_float(hiT)); }
 };
 
 // Exact divergence test of loopCalculateDiscreteModel (cudaLibrary.cu:69-71).

@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kRegThreads, 6) lle_regime_kernel(DevJob J, do
                                                                  double* scrIv, int bitWords, int sortCap,
                                                                  int* err, const long long* nDev)
 {
-    extern __shared__ unsigned smem[];
+    extern __shared__ __align__(16) unsigned smem[];
     if (nDev) J.nPoints = *nDev;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;

@@ -1,0 +1,184 @@
+// The streaming peak finder of the recorded trajectories: sample by sample, and
+// by blocks of samples.  Host and device code (the block form is compared with
+// the sample form on the CPU).
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace cbf {
+namespace {
+
+// ---------------------------------------------------------------------------
+// Streaming restatement of peakFinder (cudaLibrary.cu:220-266) over the samples
+// d[0..N) in arrival order.  Candidate i is judged when d[i+1] arrives:
+//   NORMAL : d[i] > d[i-1] (`rising`) && d[i] >= d[i+1] -> peak at i if d[i] > d[i+1],
+//            otherwise a plateau begins (inner loop of :229-246);
+//   PLATEAU: compare the plateau value with the next sample: larger -> peak at
+//            the plateau end j; smaller -> no peak; equal -> continue;
+//   SKIP   : after a peak or a rising plateau the reference sets i = j+1 and its
+//            ++i moves on to j+2, so the next arrival is not a candidate.
+// The first detected peak is dropped and intervals are (t[k+1]-t[k]) * 0.01
+// (:250-262).  NaN is absorbing for these systems, so the inner loop's
+// run-to-the-end case never yields a peak, as here.
+constexpr double kPeakIntervalUnit = 0.01;  // peakFinder's default h (cudaLibrary.cuh:204)
+
+__host__ __device__ __forceinline__ int highest_bit(unsigned v)
+{
+#ifdef __CUDA_ARCH__
+    return 31 - __clz(v);
+#else
+    return 31 - __builtin_clz(v);
+#endif
+}
+
+struct NoPeakHook {
+    __host__ __device__ __forceinline__ void operator()(double, int) const {}
+    __host__ __device__ __forceinline__ void finish(double) {}
+};
+
+// Flags of peakFinderCUDAForCalculationOfPeriodicityByOstrovsky
+// (cudaLibrary.cu:288-352) kept while the peaks stream by, over every peak:
+// non-increasing consecutive peaks (flag 0), peaks from the second on above /
+// not above the threshold (flags 1, 2), and the last recorded sample (flag 4).
+struct OstrovskyFlags {
+    double prev, last, thr;
+    bool nonInc, one, zero;
+    __host__ __device__ __forceinline__ void init(double threshold)
+    {
+        thr = threshold;
+        prev = last = 0.0;
+        nonInc = true;
+        one = zero = false;
+    }
+    __host__ __device__ __forceinline__ void operator()(double val, int k)
+    {
+        if (k >= 1) {
+            if (val - prev > 0) nonInc = false;
+            if (val > thr) one = true;
+            else zero = true;
+        }
+        prev = val;
+    }
+    __host__ __device__ __forceinline__ void finish(double sample) { last = sample; }
+};
+
+struct PeakStream {
+    double prev1, pval;  // last sample; value of the running plateau
+    int mode;            // 0 NORMAL, 1 PLATEAU, 2 SKIP
+    int rising;          // prev1 was above its predecessor
+    int detected;
+    int lastT;
+
+    __host__ __device__ __forceinline__ void init()
+    {
+        prev1 = pval = 0.0;
+        mode = rising = 0;
+        detected = 0;
+        lastT = 0;
+    }
+
+    // hook(value, k) sees every emitted peak k = 0, 1, ... (also past cap).
+    template <bool WITH_INTERVALS, class Hook>
+    __host__ __device__ __forceinline__ void emit(double val, int t, double* pk, double* iv, int cap, Hook& hook)
+    {
+        if (detected >= 1) {
+            const int k = detected - 1;
+            hook(val, k);
+            if (k < cap) {
+                pk[k] = val;
+                if (WITH_INTERVALS) iv[k] = (double)(t - lastT) * kPeakIntervalUnit;
+            }
+        }
+        lastT = t;
+        ++detected;
+    }
+
+    template <bool WITH_INTERVALS>
+    __host__ __device__ __forceinline__ void push(double v, int t, double* pk, double* iv, int cap)
+    {
+        NoPeakHook h;
+        push<WITH_INTERVALS>(v, t, pk, iv, cap, h);
+    }
+
+    template <bool WITH_INTERVALS, class Hook>
+    __host__ __device__ __forceinline__ void push(double v, int t, double* pk, double* iv, int cap, Hook& hook)
+    {
+        if (mode == 2) {
+            mode = 0;
+        } else if (mode == 1) {
+            if (pval < v) {
+                mode = 2;
+            } else if (pval > v) {
+                emit<WITH_INTERVALS>(pval, t - 1, pk, iv, cap, hook);
+                mode = 2;
+            }
+        } else if (rising && prev1 >= v) {
+            if (prev1 > v) {
+                emit<WITH_INTERVALS>(prev1, t - 1, pk, iv, cap, hook);
+                mode = 2;
+            } else {
+                mode = 1;
+                pval = prev1;
+            }
+        }
+        rising = t > 0 && v > prev1;
+        prev1 = v;
+    }
+
+    // K samples at once: the samples of times t+1 .. t+K (prev1 is time t's), all
+    // of them numbers, in ring[32 * 1] .. ring[32 * K] with time t's in ring[0];
+    // bit K-1-i of `up`: sample t+1+i is above its predecessor.  Equal to K calls
+    // of push().  A candidate arrival is one that does not rise after one that
+    // did.  The SKIP after a peak is implied -- a sample right after a descent
+    // cannot be such an arrival -- so only plateaus need the state.
+    template <int K, bool WITH_INTERVALS, class Hook>
+    __host__ __device__ __forceinline__ void push_block(unsigned up, int t, double last, const double* ring, double* pk,
+                                               double* iv, int cap, Hook& hook)
+    {
+        unsigned cand = ((((unsigned)rising << K) | up) >> 1) & ~up & ((1u << K) - 1u);
+        if (mode != 0) cand = plateau<K, WITH_INTERVALS>(mode == 2 ? -1 : 0, cand, t, ring, pk, iv, cap, hook);
+        while (cand) {
+            const int b = highest_bit(cand);
+            const int i = K - 1 - b;
+            cand &= ~(1u << b);
+            const double a = ring[32 * i], v = ring[32 * i + 32];
+            if (a > v) {
+                emit<WITH_INTERVALS>(a, t + i, pk, iv, cap, hook);
+            } else {
+                mode = 1;
+                pval = a;
+                cand = plateau<K, WITH_INTERVALS>(i + 1, cand, t, ring, pk, iv, cap, hook);
+            }
+        }
+        rising = (int)(up & 1u);
+        prev1 = last;
+    }
+
+private:
+    // Arrivals j, j+1, .. of the block against the running plateau; returns the
+    // candidates with the arrival after the plateau's end taken out (SKIP).
+    // j = -1: the plateau ended at the last arrival before the block.
+    template <int K, bool WITH_INTERVALS, class Hook>
+    __host__ __device__ unsigned plateau(int j, unsigned cand, int t, const double* ring, double* pk, double* iv, int cap,
+                                Hook& hook)
+    {
+        for (; mode == 1 && j < K; ++j) {
+            const double v = ring[32 * j + 32];
+            if (v == pval) continue;
+            if (v < pval) emit<WITH_INTERVALS>(pval, t + j, pk, iv, cap, hook);
+            mode = 2;
+            break;
+        }
+        if (mode == 2 && j + 1 < K) {
+            mode = 0;
+            cand &= ~(1u << (K - 2 - j));
+        }
+        return cand;
+    }
+
+public:
+    __host__ __device__ __forceinline__ int emitted() const { return detected > 1 ? detected - 1 : 0; }
+};
+
+}  // namespace
+}  // namespace cbf

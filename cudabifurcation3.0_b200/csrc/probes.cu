@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(256) fp64_fma_kernel(double* out, int iters, d
 // any map: each thread advances CH independent copies of the rescaled Chen step
 // at s = 1/2 (the 8-instruction form, per-thread coefficients from a ∈ [35, 36))
 // for `iters` steps and, when TRACK, folds them into the map kernels' divergence
-// trackers (two three-input maxima per pair of values).
+// trackers (one three-input maximum per pair of values).
 template <int CH, bool TRACK>
 __global__ void __launch_bounds__(128) step_chain_kernel(double* out, int iters)
 {
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(128) step_chain_kernel(double* out, int iters)
             for (int c = 0; c + 1 < CH; c += 2) tr.add2(X[c][0], X[c + 1][0]);
         }
     }
-    double s = (double)tr.s + (double)tr.u;
+    double s = (double)tr.m;
 #pragma unroll
     for (int c = 0; c < CH; ++c) s += X[c][0] + X[c][1] + X[c][2];
     if (s == -1.0) out[blockIdx.x] = s;  // never true; keeps the chains alive
