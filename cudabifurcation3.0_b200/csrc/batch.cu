@@ -68,9 +68,9 @@ __device__ __forceinline__ void bif_tile(const DevJob& J, void* out, int* aux, l
         const double* pk = slotPk + (long long)j * stride;
         int r;
         if (TASK == CBF_TASK_KDE)
-            r = kde_warp(J, pk, nj, lane);
+            r = kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
         else
-            r = dbscan_warp(J, pk, slotIv + (long long)j * stride, nj, lane, L, Sb, err, so);
+            r = dbscan_warp(dbscan_spec(J), pk, slotIv + (long long)j * stride, nj, lane, L, Sb, err, so);
         if (lane == j) res = r;
     }
     if (valid) ((int*)out)[p] = res;

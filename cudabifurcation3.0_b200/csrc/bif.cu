@@ -123,10 +123,10 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
             const double* pk = scrPeaks + (slot0 + j) * (long long)cap;
             int r;
             if (TASK == CBF_TASK_KDE) {
-                r = kde_warp(J, pk, nj, lane);
+                r = kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
             } else {
                 const double* iv = scrInt + (slot0 + j) * (long long)cap;
-                r = dbscan_warp(J, pk, iv, nj, lane, L, Sb, err, so);
+                r = dbscan_warp(dbscan_spec(J), pk, iv, nj, lane, L, Sb, err, so);
             }
             if (lane == j) res = r;
         }

@@ -66,6 +66,7 @@ __device__ __forceinline__ double sample_of(const double (&x)[S::DIM], int wv, c
 // one block: rows 0..kRing of 32 doubles (row 0: the sample before the block).
 constexpr int kRing = 16;
 constexpr int kRingWords = (kRing + 1) * 32 * 2;
+static_assert(kRingWords % 4 == 0, "every warp's shared words start on a 16-byte boundary");
 
 // What the recorded loop needs of a job.
 struct RecordSpec {
@@ -235,76 +236,312 @@ __device__ int integrate_point(const DevJob& J, long long g, double* pk, double*
 
 // ---------------------------------------------------------------------------
 // KDE mode count of one point (kde, cudaLibrary.cu:356-422), whole warp.
-__device__ int kde_warp(const DevJob& J, const double* pk, int n, int lane)
+//
+// The count is a function of the signs of d(w+1) - d(w) alone, d(w) the kernel
+// sum at sample w.  The exact sum -- FP64 differences, FP32 expf, a double
+// accumulator, the reference's peak order -- costs about 50 issue cycles a term
+// (six FP64 instructions and two conversions to and from double, which run at a
+// quarter of that rate), and made the map's epilogue three times its integration
+// (331 ms of 440 for the 1024^2 Lorenz map with 4 samples per peak).  So the signs
+// are first settled by FP32 sums with an error bound (kde_fast_sum: one
+// subtraction, one square, one ex2 and one addition a term), over peaks sorted
+// once per point so that a chunk of samples meets one window of them; a pair of
+// samples whose difference is within the two bounds is settled by the exact
+// sums (the same map: 440 -> 302 ms; a point takes 27 chunks and 1400 FP32 terms
+// instead of 50 and 7000 exact ones).  Windows of 6 bandwidths first (what lies outside adds at most e^-18 a
+// peak), of 16 next (outside, the exact terms are +0 too), the exact sums last.
+constexpr int kKdeSortCap = 1024;  // peaks a warp sorts (its ring words hold them)
+constexpr double kKdeNear = 6.0, kKdeFar = 16.0;         // window half-widths in bandwidths
+constexpr double kKdeScale = 0.84932180028801904;       // sqrt(log2(e) / 2)
+constexpr float kKdeDropped = 1.6e-8f;                  // above e^(-kKdeNear^2 / 2)
+
+// The exact sum at this lane's sample `delt`, the warp's samples lying in
+// [dlo, dhi].  Rounded subtraction is monotone, so a peak with fl(p - dhi) > skip
+// or fl(p - dlo) < -skip has |fl(p - delt)| > skip for every lane, i.e. it adds
+// exactly +0 everywhere.  One ballot per 32 peaks drops those; the rest are summed
+// in ascending m.  A NaN bound fails both comparisons and keeps every peak.
+__device__ __noinline__ double kde_exact_sum(const double* pk, int n, double delt, double dlo, double dhi,
+                                             double skip, double H, double invH, bool active, int lane)
 {
+    double d2 = 0;
+    for (int g = 0; g < n; g += 32) {
+        const int m = g + lane;
+        const double pv = m < n ? pk[m] : 0.0;
+        const bool near = m < n && !(pv - dhi > skip) && !(pv - dlo < -skip);
+        unsigned mask = __ballot_sync(kFull, near);
+        while (mask) {
+            const int j = __ffs(mask) - 1;
+            mask &= mask - 1;
+            const double dd = __shfl_sync(kFull, pv, j) - delt;
+            // |dd| > 16|H| makes the FP32 exponent argument <= -128, where expf
+            // is exactly +0 (checked exhaustively on the device by
+            // cbf_probe_expf_zero), and adding +0 leaves the sum unchanged.
+            if (active && !(fabs(dd) > skip)) {
+                const double tmp = invH != 0.0 ? dd * invH : dd / H;
+                d2 += (double)expf((float)(-((tmp * tmp) / 2)));
+            }
+        }
+    }
+    return d2;
+}
+
+// Peaks of one point as sorted floats: key[i] = (p - mid) * scale in ascending
+// order, scale = kKdeScale / |H| (so a term is 2^-(key - x)^2), padded with +inf
+// to P, a power of two >= 32.
+struct KdeSorted {
+    const float* key;
+    int n;
+    double mid, scale;
+    float qmax;   // largest |key|
+    float weight; // peaks per key
+};
+
+// Sorts the peaks into key[0..P) (shared); false where the FP32 sums would not
+// do: not every value finite, or keys too large for the bound to be of use.
+__device__ bool kde_sort(float* key, const double* pk, int n, double H, int lane, KdeSorted& ks)
+{
+    double lo = INFINITY, hi = -INFINITY;
+    bool bad = false;
+    for (int m = lane; m < n; m += 32) {
+        const double v = pk[m];
+        bad |= !isfinite(v);
+        lo = fmin(lo, v);
+        hi = fmax(hi, v);
+    }
+    if (__any_sync(kFull, bad)) return false;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(kFull, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(kFull, hi, o));
+    }
+    ks.n = n;
+    ks.key = key;
+    ks.mid = lo + (hi - lo) * 0.5;
+    ks.scale = kKdeScale / fabs(H);
+    const double span = (hi - lo) * ks.scale;
+    if (!(span < 1e5) || !(fabs(ks.mid) < 1e100)) return false;
+    ks.qmax = (float)(span * 0.5) * 1.001f + 1e-6f;
+    ks.weight = 1.0f;
+    int P = 32;
+    __syncwarp();
+    if (span < 0x1p-18) {
+        // one value but for its last bits (a fixed point's wobble, thousands of
+        // peaks): one key of weight n; |key - 0| <= qmax enters the bound
+        key[lane] = lane == 0 ? 0.0f : INFINITY;
+        ks.n = 1;
+        ks.weight = (float)n;
+        __syncwarp();
+        return true;
+    }
+    while (P < n) P <<= 1;
+    for (int m = lane; m < P; m += 32) key[m] = m < n ? (float)((pk[m] - ks.mid) * ks.scale) : INFINITY;
+    __syncwarp();
+    for (int size = 2; size <= P; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int t = lane; t < (P >> 1); t += 32) {
+                const int i = 2 * t - (t & (stride - 1));
+                const float ki = key[i], kj = key[i + stride];
+                const float mn = fminf(ki, kj), mx = fmaxf(ki, kj);
+                const bool up = (i & size) == 0;
+                key[i] = up ? mn : mx;
+                key[i + stride] = up ? mx : mn;
+            }
+            __syncwarp();
+        }
+    }
+    return true;
+}
+
+// Keys below x among key[0..n), whole warp: the last key of each of 32 segments,
+// then the same within the first segment whose last key is not below.
+__device__ __forceinline__ int kde_below(const KdeSorted& ks, float x, int lane)
+{
+    int at = 0, len = ks.n;
+    for (;;) {
+        const int seg = (len + 31) >> 5;
+        const int end = min((lane + 1) * seg, len);  // of this lane's segment, if not empty
+        const bool below = lane * seg < len && ks.key[at + end - 1] < x;
+        const int c = __popc(__ballot_sync(kFull, below)) * seg;
+        if (seg == 1 || c >= len) return at + min(c, len);
+        at += c;
+        len = min(seg, len - c);
+    }
+}
+
+__device__ __forceinline__ float ex2_ftz(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The FP32 sum at x over the peaks of key[lo..hi) (and up to three on either
+// side, +inf among them: true terms, or 0), four at a time; *least: the smallest
+// squared distance met.
+__device__ __forceinline__ float kde_fast_sum(const KdeSorted& ks, int lo, int hi, float x, float* least)
+{
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, s0 = INFINITY, s1 = INFINITY;
+    for (int m = lo & ~3; m < hi; m += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(ks.key + m);
+        const float u0 = q.x - x, u1 = q.y - x, u2 = q.z - x, u3 = q.w - x;
+        const float v0 = u0 * u0, v1 = u1 * u1, v2 = u2 * u2, v3 = u3 * u3;
+        s0 = fminf(s0, fminf(v0, v1));
+        s1 = fminf(s1, fminf(v2, v3));
+        a0 += ex2_ftz(-v0);
+        a1 += ex2_ftz(-v1);
+        a2 += ex2_ftz(-v2);
+        a3 += ex2_ftz(-v3);
+    }
+    *least = fminf(s0, s1);
+    return (a0 + a1) + (a2 + a3);
+}
+
+// Bound of |fast sum - exact sum| relative to the sum, for `terms` terms with
+// |key - x| <= U, |key| <= Q, |x| <= X, in units of 2^-24:
+//   key and x are rounded (Q + X), so is their difference (U), and a key of
+//   weight n lies within 64 units of its peaks: the exponent u^2 is off by
+//   2U(Q + X + U + 64) and its own rounding U^2; the exact exponent is rounded to
+//   FP32 (U^2); ln 2 times that, plus 2^-22 for ex2.approx and 2 ulp for expf
+//   (4 + 4), and the additions of four partial sums.
+// Terms with U^2 > 126 are at most 2^-126 on either side (absolute bound).
+__device__ __forceinline__ float kde_rel_bound(float U, float Q, float X, int terms, float spread)
+{
+    U = fminf(U, 11.3f);
+    const float e = 0.6932f * (2.0f * U * (Q + X + U + spread) + 2.0f * U * U) + 8.0f + 0.25f * (float)terms + 4.0f;
+    return 1.05f * 0x1p-24f * e;
+}
+
+// What the KDE epilogue needs of a job.
+struct KdeSpec {
+    double i1, i2, H, skip, invH;
+    int maxPeaks, sampling, fixed;
+};
+
+__device__ __forceinline__ KdeSpec kde_spec(const DevJob& J)
+{
+    return KdeSpec{J.kdeI1, J.kdeI2, J.kdeH, J.kdeSkip, J.kdeInvH, J.maxPeaks, J.kdeSampling, J.kdeFixed};
+}
+
+// `keys`: room for keyCap floats of this warp, a power of two >= 32, 16-byte
+// aligned; in shared memory (SHARED) or in global memory.  A function of its own,
+// like the recorded loop: its registers are not the integration's.
+template <bool SHARED>
+__device__ __noinline__ int kde_warp(const KdeSpec J, const double* pk, int n, int lane, float* keys, int keyCap)
+{
+    float* key = SHARED ? static_cast<float*>(__cvta_shared_to_generic(__cvta_generic_to_shared(keys))) : keys;
     if (n == 0) return 0;
     if (n == 1 || n == 2) return 1;
     if (n > J.maxPeaks) return J.maxPeaks;
 
-    const double k1 = J.kdeFixed ? (double)J.kdeSampling : (double)(J.kdeSampling * n);
-    const double k2 = (J.kdeI2 - J.kdeI1) / (k1 - 1);
+    const double k1 = J.fixed ? (double)J.sampling : (double)(J.sampling * n);
+    const double k2 = (J.i2 - J.i1) / (k1 - 1);
     // `for (int w = 0; w < k1 - 1; ++w)`: k1 is integral, so W = k1 - 1 iterations.
     const int W = (k1 - 1 > 0) ? (int)ceil(k1 - 1) : 0;
-    const double skip = J.kdeSkip;
-    const double H = J.kdeH;
-    const double invH = J.kdeInvH;
+    const double skip = J.skip, H = J.H, invH = J.invH;
 
-    double pp = 0, pr = 0, cur = 0;
-    bool strange = false;
+    // FP32 sums where they can decide: a usable bandwidth and interval, no more
+    // peaks than a warp sorts, and a bound of their error well below 1.
+    KdeSorted ks;
+    bool fast = n <= keyCap && W > 2 && fabs(H) > 1e-30 && fabs(H) < 1e30 && fabs(J.i1) < 1e100 &&
+                fabs(J.i2) < 1e100 && k2 != 0 && kde_sort(key, pk, n, H, lane, ks);
+    float width = 0.f, spread = 0.f;  // a chunk's extent, and a key's, in key units
+    if (fast) {
+        width = (float)(31.0 * fabs(k2) * ks.scale);
+        spread = ks.n == 1 ? 64.0f : 0.0f;  // 2^-18 in units of 2^-24
+        fast = kde_rel_bound(11.3f, ks.qmax, ks.qmax + 14.0f + width, n, spread) < 0x1p-6f;
+    }
+
     int res = 0;
-    for (int base = 0; base < W; base += 32) {
+    bool prevUp = false, strange = false, lastUp = false;
+    // Samples in chunks of 32, each starting with its predecessor's last: pairs
+    // (lane, lane + 1) for lane < cnt - 1.
+    for (int base = 0; base < W - 1 || base == 0; base += 31) {
+        if (W == 0) break;
         const int w = base + lane;
         const int cnt = min(32, W - base);
-        const double delt = w * k2 + J.kdeI1;
-        // delt is monotone in w (rounded products and sums are), so the chunk's
-        // samples lie in [dlo, dhi], and rounded subtraction is monotone too: a
-        // peak with fl(p - dhi) > skip or fl(p - dlo) < -skip has |fl(p - delt)|
-        // > skip for every lane, i.e. it adds exactly +0 everywhere.  One ballot
-        // per 32 peaks drops those; the rest are summed in ascending m as before.
-        // A NaN bound fails both comparisons and keeps every peak.
+        const double delt = w * k2 + J.i1;
+        // delt is monotone in w (rounded products and sums are)
         const double dFirst = __shfl_sync(kFull, delt, 0);
         const double dLast = __shfl_sync(kFull, delt, cnt - 1);
         const double dlo = k2 >= 0 ? dFirst : dLast;
         const double dhi = k2 >= 0 ? dLast : dFirst;
-        double d2 = 0;
-        for (int g = 0; g < n; g += 32) {
-            const int m = g + lane;
-            const double pv = m < n ? pk[m] : 0.0;
-            const bool near = m < n && !(pv - dhi > skip) && !(pv - dlo < -skip);
-            unsigned mask = __ballot_sync(kFull, near);
-            while (mask) {
-                const int j = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const double dd = __shfl_sync(kFull, pv, j) - delt;
-                // |dd| > 16|H| makes the FP32 exponent argument <= -128, where expf
-                // is exactly +0 (checked exhaustively on the device by
-                // cbf_probe_expf_zero), and adding +0 leaves the sum unchanged.
-                if (w < W && !(fabs(dd) > skip)) {
-                    const double tmp = invH != 0.0 ? dd * invH : dd / H;
-                    d2 += (double)expf((float)(-((tmp * tmp) / 2)));
+        const bool pair = lane < cnt - 1;
+        bool up = false, eq = false;
+        unsigned open = cnt > 1 ? (0xffffffffu >> (33 - cnt)) : 0u;  // pairs whose sign is not settled
+        if (fast) {
+            const float x = (float)((delt - ks.mid) * ks.scale);
+            const float xlo = (float)((dlo - ks.mid) * ks.scale), xhi = (float)((dhi - ks.mid) * ks.scale);
+            // beyond 16 bandwidths (and the roundings of key and x) of every
+            // peak the exact sums are +0: all equal
+            const float reach = (float)(kKdeFar * kKdeScale) + 0.05f;
+            if (fmaxf(-ks.qmax - xhi, xlo - ks.qmax) > reach) {
+                eq = pair;
+                open = 0;
+            }
+#pragma unroll 1
+            for (int tier = 0; tier < 2 && open; ++tier) {
+                const float half = tier == 0 ? (float)(kKdeNear * kKdeScale) : reach;
+                const int lo = kde_below(ks, xlo - half, lane);
+                const int hi = kde_below(ks, xhi + half, lane);
+                float least;
+                const float a = kde_fast_sum(ks, lo, hi, x, &least) * ks.weight;
+                float e = a * kde_rel_bound(half + width + 1.0f, ks.qmax, ks.qmax + 14.0f + width, hi - lo + 6, spread) +
+                          (float)n * 0x1p-125f;
+                if (tier == 0) e += (float)(ks.n - (hi - lo)) * ks.weight * kKdeDropped;
+                else if (least > reach * reach) e = 0.f;  // no peak in reach: +0, exactly
+                const float an = __shfl_down_sync(kFull, a, 1), en = __shfl_down_sync(kFull, e, 1);
+                up = an > a;
+                eq = a == 0.f && an == 0.f && e == 0.f && en == 0.f;
+                // 1.0001: the roundings of e + en and an - a themselves
+                const bool sure = eq || fabsf(an - a) > (e + en) * 1.0001f;
+                open = __ballot_sync(kFull, pair && !sure);
+            }
+        }
+        bool nan = false;
+        if (open || W == 1) {
+            // exact sums of the samples of open pairs
+            const unsigned act = W == 1 ? 1u : open | (open << 1);
+            const double d0 = __shfl_sync(kFull, delt, __ffs(act) - 1);
+            const double d1 = __shfl_sync(kFull, delt, highest_bit(act));
+            const double d = kde_exact_sum(pk, n, delt, k2 >= 0 ? d0 : d1, k2 >= 0 ? d1 : d0, skip, H, invH,
+                                           (act >> lane) & 1u, lane);
+            const double dn = __shfl_down_sync(kFull, d, 1);
+            if ((open >> lane) & 1u) {
+                up = dn > d;
+                eq = dn == d;
+                nan = !(up || eq || dn < d);
+            }
+            if (W == 1) lastUp = __shfl_sync(kFull, d, 0) > 0;
+        }
+        const unsigned pm = cnt > 1 ? (0xffffffffu >> (33 - cnt)) : 0u;
+        const unsigned U = __ballot_sync(kFull, up && pair), E = __ballot_sync(kFull, eq && pair);
+        const unsigned N = __ballot_sync(kFull, nan && pair);
+        if (cnt <= 1) break;
+        if (!(E | N) && !strange) {
+            // maxima: a rise and then a descent
+            res += __popc(((U << 1) | (prevUp ? 1u : 0u)) & ~U & pm);
+            prevUp = (U >> (cnt - 2)) & 1u;
+        } else if (E == pm) {  // level throughout
+            strange |= prevUp;
+            prevUp = false;
+        } else {
+            // the reference's plateau states, pair by pair
+            for (int j = 0; j < cnt - 1; ++j) {
+                const bool u = (U >> j) & 1u, q = (E >> j) & 1u, d = !u && !q && !((N >> j) & 1u);
+                if (strange) {
+                    if (u) strange = false;
+                    else if (d) { strange = false; ++res; }
+                } else if (prevUp && d) {
+                    ++res;
+                } else if (prevUp && q) {
+                    strange = true;
                 }
+                prevUp = u;
             }
         }
-        for (int j = 0; j < cnt; ++j) {
-            const double val = __shfl_sync(kFull, d2, j);
-            pp = pr;
-            pr = cur;
-            cur = val;
-            if (base + j < 2) continue;
-            if (strange) {
-                if (pr == cur) continue;
-                else if (pr < cur) { strange = false; continue; }
-                else if (pr > cur) { strange = false; ++res; continue; }
-            } else if (pr > pp && pr > cur) {
-                ++res;
-                continue;
-            } else if (pr > pp && pr == cur) {
-                strange = true;
-                continue;
-            }
-        }
+        lastUp = prevUp;
     }
-    if (pr < cur) ++res;
+    if (lastUp) ++res;
     return res;
 }
 
@@ -347,11 +584,12 @@ struct DbscanSort {
 
 // 32-bit words of shared memory per warp: the bitsets L and S of `bitWords`
 // words each, and with `sortCap` > 0 (a power of two, 32..1024) also E, D and
-// the sort keys.  The recorded loop's ring lies in the same words (a warp's
-// epilogues start when all its lanes have integrated).
+// the sort keys.  The recorded loop's ring and the KDE epilogue's sorted peaks lie
+// in the same words (a warp's epilogues start when all its lanes have integrated).
+// A multiple of four words: every warp's start is 16-byte aligned.
 __host__ __device__ inline int dbscan_warp_words(int bitWords, int sortCap)
 {
-    const int w = sortCap > 0 ? 4 * bitWords + sortCap : 2 * bitWords;
+    const int w = ((sortCap > 0 ? 4 * bitWords + sortCap : 2 * bitWords) + 3) & ~3;
     return w > kRingWords ? w : kRingWords;
 }
 
@@ -607,11 +845,19 @@ __device__ int2 dbscan_open_run(unsigned* L, int i, int j, int M, int lane)
     return make_int2(opened, openedScanned);
 }
 
+// What the DBSCAN epilogue needs of a job.
+struct DbscanSpec {
+    double dbEps, dbSkip;
+    int maxPeaks;
+};
+
+__device__ __forceinline__ DbscanSpec dbscan_spec(const DevJob& J) { return DbscanSpec{J.dbEps, J.dbSkip, J.maxPeaks}; }
+
 // DBSCAN cluster count of one point; `so` (shared memory of this warp) enables
 // the sorted path for points with n - 1 <= so.cap peaks.
-__device__ int dbscan_warp(const DevJob& J, const double* pk,
-                           const double* iv, int n, int lane, unsigned* L,
-                           unsigned* Sb, int* err, DbscanSort so = DbscanSort())
+__device__ __noinline__ int dbscan_warp(const DbscanSpec J, const double* pk,
+                                        const double* iv, int n, int lane, unsigned* L,
+                                        unsigned* Sb, int* err, DbscanSort so)
 {
     if (n <= 0) return 0;
     if (n == 1) return 1;

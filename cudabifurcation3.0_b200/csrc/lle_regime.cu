@@ -137,7 +137,7 @@ __device__ __forceinline__ int regime_tile(const DevJob& J, long long g, bool va
         else {
             const double* pk = scrPk + (slot0 + j) * (long long)cap;
             const double* iv = scrIv + (slot0 + j) * (long long)cap;
-            r = min(dbscan_warp(J, pk, iv, nj, lane, L, Sb, err, so), kNumClasses - 1);
+            r = min(dbscan_warp(dbscan_spec(J), pk, iv, nj, lane, L, Sb, err, so), kNumClasses - 1);
         }
         if (lane == j) res = r;
     }
