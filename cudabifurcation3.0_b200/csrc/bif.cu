@@ -18,7 +18,16 @@
 //             in shared memory; the inner neighbour loop over k is a ballot
 //             (its iterations are independent in the reference), popcount
 //             updates the neighbour counter.
-// Results leave as one coalesced 32-wide store per warp.
+// Results leave as one coalesced store per tile.
+//
+// Tiles are taken from a device counter: how long a point's epilogue takes
+// depends on its peaks, and a fixed assignment left the warps with few of them
+// idle at the end.  A tile holds 32 points where the map fills the GPU and fewer
+// where it does not (tile_points): the steps of a warp's lanes run together, its
+// epilogues one after the other.  Lorenz 1024^2: KDE map 302 -> 188 ms, DBSCAN map
+// 207 -> 156 ms; where points of very many peaks reach the second pass (recorded
+// variable z) 1152 -> 167 ms: a few dozen warps used to do all of them.
+#include <algorithm>
 #include <type_traits>
 
 #include "bif_device.cuh"
@@ -60,30 +69,48 @@ struct Overflow {
 template <class S>
 constexpr int kBifMinBlocks = S::DIM == 3 ? 8 : 4;
 
+// Scratch of a launch: peak slots (and intervals) of `tile` points per warp, the
+// tile counter, and per warp `keyCap` floats for the KDE epilogue's sorted peaks
+// where the shared memory does not hold them (0: none).
+struct BifScratch {
+    double* peaks;
+    double* intervals;
+    unsigned long long* queue;
+    float* keys;
+    int keyCap;
+    int* err;
+};
+
 template <class S, int TASK>
 __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(const DevJob J, void* __restrict__ d_out,
-                                                          int* __restrict__ d_aux,
-                                                          double* scrPeaks,
-                                                          double* scrInt,
-                                                          int bitWords, int sortCap,
-                                                          int* __restrict__ err, const Overflow ov)
+                                                                            int* __restrict__ d_aux,
+                                                                            const BifScratch sc, int bitWords,
+                                                                            int sortCap, int tilePts,
+                                                                            const Overflow ov)
 {
     extern __shared__ __align__(16) unsigned smem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const long long warpId = (long long)blockIdx.x * kBifWarps + wib;
     const long long nWarps = (long long)gridDim.x * kBifWarps;
-    const long long nTiles = (J.nPoints + 31) / 32;
+    const long long nTiles = (J.nPoints + tilePts - 1) / tilePts;
     const int cap = J.peakCap;
     unsigned* L = smem + (size_t)wib * dbscan_warp_words(bitWords, sortCap);
     unsigned* Sb = L + bitWords;
     const DbscanSort so = dbscan_sort_area(L, bitWords, sortCap);
     double* ring = ring_column(L, lane);
 
-    for (long long tile = warpId; tile < nTiles; tile += nWarps) {
-        const long long p = tile * 32 + lane;
-        const bool valid = p < J.nPoints;
-        const long long g = grid_index(J, p);
+    for (long long next = warpId;; next += nWarps) {
+        long long tile = next;
+        if (sc.queue) {
+            unsigned long long t = 0;
+            if (lane == 0) t = atomicAdd(sc.queue, 1ull);
+            tile = (long long)__shfl_sync(kFull, t, 0);
+        }
+        if (tile >= nTiles) break;
+        const long long p = tile * tilePts + lane;
+        const bool valid = lane < tilePts && p < J.nPoints;
+        const long long g = valid ? grid_index(J, p) : 0;
 
         if (TASK == CBF_TASK_PEAKS) {
             if (valid) {
@@ -100,9 +127,9 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
             continue;
         }
 
-        const long long slot0 = warpId * 32;
-        double* myPk = scrPeaks + (slot0 + lane) * (long long)cap;
-        double* myIv = task_with_intervals(TASK) ? scrInt + (slot0 + lane) * (long long)cap : nullptr;
+        const long long slot0 = warpId * tilePts;
+        double* myPk = sc.peaks + (slot0 + lane) * (long long)cap;
+        double* myIv = task_with_intervals(TASK) ? sc.intervals + (slot0 + lane) * (long long)cap : nullptr;
         int n = 0, div = 0;
         OstrovskyFlags of;
         of.init(J.ostThr);
@@ -117,16 +144,18 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
         __syncwarp();
 
         int res = 0;
-        const int live = (int)min(32ll, J.nPoints - tile * 32);
+        const int live = (int)min((long long)tilePts, J.nPoints - tile * tilePts);
         for (int j = 0; j < live; ++j) {
             const int nj = __shfl_sync(kFull, over ? 0 : n, j);
-            const double* pk = scrPeaks + (slot0 + j) * (long long)cap;
+            const double* pk = sc.peaks + (slot0 + j) * (long long)cap;
             int r;
             if (TASK == CBF_TASK_KDE) {
-                r = kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
+                r = sc.keyCap > 0
+                        ? kde_warp<false>(kde_spec(J), pk, nj, lane, sc.keys + warpId * sc.keyCap, sc.keyCap)
+                        : kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
             } else {
-                const double* iv = scrInt + (slot0 + j) * (long long)cap;
-                r = dbscan_warp(dbscan_spec(J), pk, iv, nj, lane, L, Sb, err, so);
+                const double* iv = sc.intervals + (slot0 + j) * (long long)cap;
+                r = dbscan_warp(dbscan_spec(J), pk, iv, nj, lane, L, Sb, sc.err, so);
             }
             if (lane == j) res = r;
         }
@@ -148,63 +177,96 @@ __global__ void scatter_kernel(const T* __restrict__ src, const long long* __res
     if (k < n) dst[slot[k]] = src[k];
 }
 
-// One launch of the fused kernel over the job's points (synchronises `s`).
-template <class S, int TASK>
-cudaError_t bif_pass(const DevJob& J, void* d_out, int* d_aux, const Overflow& ov, cudaStream_t s)
+// Points per tile of a map of n points: 32, or fewer where that leaves less than
+// four warps for each of the SMs' four schedulers.  Up to three warps a scheduler
+// the integration is bound by the latency of a lane's own chain (65 cycles a
+// step, of which a warp issues 22), so it costs no more when fewer lanes of a
+// warp are in use, and the epilogues of a tile -- serial within a warp -- spread
+// over more warps (at four warps a step takes 90 cycles; with eight, 180).
+int tile_points(long long n, int sms)
 {
-    const long long nTiles = (J.nPoints + 31) / 32;
-    if (nTiles == 0) return cudaSuccess;
-    const bool needScratch = (TASK == CBF_TASK_KDE || task_with_intervals(TASK));
-    const int bitWords = task_with_intervals(TASK) ? (J.peakCap + 31) / 32 : 0;
-    const int sortCap = bif_sort_cap(TASK, J.peakCap);
-    const size_t smemBytes = (size_t)kBifWarps * dbscan_warp_words(bitWords, sortCap) * sizeof(unsigned);
+    const long long t = (n + 16ll * sms - 1) / (16ll * sms);
+    return (int)std::min(32ll, std::max(1ll, t));
+}
 
+// Shape of one launch.
+struct BifShape {
+    int bitWords, sortCap, tile, keyCap;
+    size_t smem;
+    long long blocks;      // one per resident slot, or fewer
+    size_t peakBytes;      // peak slots of a block
+    size_t blockBytes;     // ... and its sorted keys
+};
+
+template <class S, int TASK>
+cudaError_t bif_shape(const DevJob& J, int maxTile, bool keys, BifShape* sh)
+{
     auto kern = bif_kernel<S, TASK>;
+    sh->bitWords = task_with_intervals(TASK) ? (J.peakCap + 31) / 32 : 0;
+    sh->sortCap = bif_sort_cap(TASK, J.peakCap);
+    sh->smem = (size_t)kBifWarps * dbscan_warp_words(sh->bitWords, sh->sortCap) * sizeof(unsigned);
     cudaError_t e;
-    if (smemBytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes);
+    if (sh->smem > 48 * 1024) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh->smem);
         if (e != cudaSuccess) return e;
     }
     int dev = 0, sms = 0, perSm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kBifThreads, smemBytes)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kBifThreads, sh->smem)) != cudaSuccess)
         return e;
     if (perSm < 1) return cudaErrorInvalidConfiguration;
+    sh->tile = std::min(maxTile, tile_points(J.nPoints, sms));
+    const long long nTiles = (J.nPoints + sh->tile - 1) / sh->tile;
+    sh->blocks = std::min((nTiles + kBifWarps - 1) / kBifWarps, (long long)sms * perSm);
+    sh->peakBytes = (size_t)kBifWarps * sh->tile * J.peakCap * sizeof(double) * (task_with_intervals(TASK) ? 2 : 1);
+    sh->keyCap = 0;
+    if (keys && TASK == CBF_TASK_KDE && J.peakCap > kKdeSortCap) {
+        sh->keyCap = kKdeSortCap;
+        while (sh->keyCap < J.peakCap && sh->keyCap < (1 << 20)) sh->keyCap <<= 1;
+    }
+    sh->blockBytes = sh->peakBytes + (size_t)kBifWarps * sh->keyCap * sizeof(float);
+    return cudaSuccess;
+}
 
-    long long blocks = (nTiles + kBifWarps - 1) / kBifWarps;
-    const long long resident = (long long)sms * perSm;
-    if (blocks > resident) blocks = resident;
-
-    double* scrPeaks = nullptr;
-    double* scrInt = nullptr;
-    int* err = nullptr;
+// One launch of the fused kernel over the job's points (synchronises `s` where
+// it takes scratch).
+template <class S, int TASK>
+cudaError_t bif_pass(const DevJob& J, void* d_out, int* d_aux, const Overflow& ov, cudaStream_t s)
+{
+    if (J.nPoints == 0) return cudaSuccess;
+    const bool needScratch = (TASK == CBF_TASK_KDE || task_with_intervals(TASK));
+    BifShape sh;
+    cudaError_t e = bif_shape<S, TASK>(J, 32, true, &sh);
+    if (e != cudaSuccess) return e;
+    BifScratch sc{};
+    char* mem = nullptr;
     if (needScratch) {
-        // Per-warp scratch: 32 points x cap peaks (x2 with intervals).  Bound it.
-        const size_t perBlock = (size_t)kBifThreads * J.peakCap * sizeof(double) *
-                                (task_with_intervals(TASK) ? 2 : 1);
         size_t freeB = 0, totalB = 0;
         if ((e = cudaMemGetInfo(&freeB, &totalB)) != cudaSuccess) return e;
-        size_t budget = freeB / 4;
-        const size_t cap8 = (size_t)8 << 30;
-        if (budget > cap8) budget = cap8;
-        long long fit = (long long)(budget / perBlock);
-        if (fit < 1) fit = 1;
-        if (blocks > fit) blocks = fit;
-        const size_t bytes = (size_t)blocks * perBlock;
-        if ((e = cudaMallocAsync((void**)&scrPeaks, bytes + 256, s)) != cudaSuccess) return e;
-        if (task_with_intervals(TASK)) scrInt = scrPeaks + (size_t)blocks * kBifThreads * J.peakCap;
-        err = (int*)((char*)scrPeaks + bytes);
-        if ((e = cudaMemsetAsync(err, 0, sizeof(int), s)) != cudaSuccess) return e;
+        const size_t budget = std::min(freeB / 4, (size_t)8 << 30);
+        sh.blocks = std::min(sh.blocks, std::max(1ll, (long long)(budget / sh.blockBytes)));
+        // [error flag, counter | peaks | intervals | keys]
+        if ((e = cudaMallocAsync((void**)&mem, 256 + (size_t)sh.blocks * sh.blockBytes, s)) != cudaSuccess) return e;
+        sc.err = (int*)mem;
+        sc.queue = (unsigned long long*)(mem + 128);
+        sc.peaks = (double*)(mem + 256);
+        if (task_with_intervals(TASK)) sc.intervals = sc.peaks + (size_t)sh.blocks * kBifWarps * sh.tile * J.peakCap;
+        sc.keys = (float*)(mem + 256 + (size_t)sh.blocks * sh.peakBytes);
+        sc.keyCap = sh.keyCap;
+        if ((e = cudaMemsetAsync(mem, 0, 256, s)) != cudaSuccess) {
+            cudaFreeAsync(mem, s);
+            return e;
+        }
     }
-    kern<<<(unsigned)blocks, kBifThreads, smemBytes, s>>>(J, d_out, d_aux, scrPeaks, scrInt, bitWords, sortCap,
-                                                          err, ov);
+    bif_kernel<S, TASK><<<(unsigned)sh.blocks, kBifThreads, sh.smem, s>>>(J, d_out, d_aux, sc, sh.bitWords, sh.sortCap,
+                                                                          sh.tile, ov);
     note_launch();
     e = cudaGetLastError();
     if (needScratch) {
         int hostErr = 0;
-        cudaError_t e2 = cudaMemcpyAsync(&hostErr, err, sizeof(int), cudaMemcpyDeviceToHost, s);
-        cudaError_t e3 = cudaFreeAsync(scrPeaks, s);
+        cudaError_t e2 = cudaMemcpyAsync(&hostErr, sc.err, sizeof(int), cudaMemcpyDeviceToHost, s);
+        cudaError_t e3 = cudaFreeAsync(mem, s);
         if (e == cudaSuccess) e = e2;
         if (e == cudaSuccess) e = e3;
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -275,39 +337,34 @@ cudaError_t launch_bif_s(const DevJob& J, void* d_out, int* d_aux, cudaStream_t 
 }
 
 // One pass of the fused kernel with caller-provided scratch (no allocation);
-// synchronises `s` to read the error flag.
+// synchronises `s` to read the error flag.  The tile counter takes the first 256
+// bytes; where the scratch holds the lanes of few warps, tiles are smaller
+// (more warps share it).
 template <class S, int TASK>
 cudaError_t prealloc_pass(const DevJob& J, void* d_out, double* scratch, size_t scratchBytes, int* err,
                           const Overflow& ov, cudaStream_t s)
 {
-    const long long nTiles = (J.nPoints + 31) / 32;
-    if (nTiles == 0) return cudaSuccess;
-    const int bitWords = (TASK == CBF_TASK_DBSCAN) ? (J.peakCap + 31) / 32 : 0;
-    const int sortCap = bif_sort_cap(TASK, J.peakCap);
-    const size_t smemBytes = (size_t)kBifWarps * dbscan_warp_words(bitWords, sortCap) * sizeof(unsigned);
-    auto kern = bif_kernel<S, TASK>;
+    if (J.nPoints == 0) return cudaSuccess;
+    const size_t perLane = (size_t)J.peakCap * sizeof(double) * (task_with_intervals(TASK) ? 2 : 1);
+    if (scratchBytes < 256 + kBifWarps * perLane) return cudaErrorInvalidValue;
+    const size_t peakBytes = scratchBytes - 256;
+    int dev = 0, sms = 0;
     cudaError_t e;
-    if (smemBytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes);
-        if (e != cudaSuccess) return e;
-    }
-    int dev = 0, sms = 0, perSm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kBifThreads, smemBytes)) != cudaSuccess)
-        return e;
-    if (perSm < 1) return cudaErrorInvalidConfiguration;
-    const size_t perBlock = (size_t)kBifThreads * J.peakCap * sizeof(double) *
-                            (task_with_intervals(TASK) ? 2 : 1);
-    long long blocks = (nTiles + kBifWarps - 1) / kBifWarps;
-    const long long resident = (long long)sms * perSm;
-    if (blocks > resident) blocks = resident;
-    const long long fit = (long long)(scratchBytes / perBlock);
-    if (fit < 1) return cudaErrorInvalidValue;
-    if (blocks > fit) blocks = fit;
-    double* scrInt = (TASK == CBF_TASK_DBSCAN) ? scratch + (size_t)blocks * kBifThreads * J.peakCap : nullptr;
-    kern<<<(unsigned)blocks, kBifThreads, smemBytes, s>>>(J, d_out, nullptr, scratch, scrInt, bitWords, sortCap,
-                                                          err, ov);
+    const long long lanes = (long long)(peakBytes / perLane);
+    BifShape sh;
+    if ((e = bif_shape<S, TASK>(J, tile_points(2 * lanes, sms), false, &sh)) != cudaSuccess) return e;
+    sh.blocks = std::min(sh.blocks, (long long)(peakBytes / sh.peakBytes));
+    if (sh.blocks < 1) return cudaErrorInvalidValue;
+    BifScratch sc{};
+    sc.err = err;
+    sc.queue = (unsigned long long*)scratch;
+    sc.peaks = scratch + 32;
+    if (task_with_intervals(TASK)) sc.intervals = sc.peaks + (size_t)sh.blocks * kBifWarps * sh.tile * J.peakCap;
+    if ((e = cudaMemsetAsync(sc.queue, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    bif_kernel<S, TASK><<<(unsigned)sh.blocks, kBifThreads, sh.smem, s>>>(J, d_out, nullptr, sc, sh.bitWords, sh.sortCap,
+                                                                          sh.tile, ov);
     note_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int hostErr = 0;
