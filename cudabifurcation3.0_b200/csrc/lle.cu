@@ -14,10 +14,16 @@
 // stops that integration at the first violation (loopCalculateDiscreteModel,
 // cudaLibrary.cu:69-71).  Here each renormalisation interval first runs
 // unchecked while folding the high word of |x[0]| and |y[0]| into a running
-// integer max (ALU pipe, off the FP64 pipe); only if that max reaches the high
-// word of the exact threshold is the interval replayed from a register snapshot
-// with the exact per-step check.  Results are identical; the common case pays
-// two integer ops per step.
+// maximum (one three-input FP32 maximum for both); only if that max reaches the
+// high word of the exact threshold is the interval replayed from a register
+// snapshot with the exact per-step check.  Results are identical.
+//
+// Bound: the register reads of the FP64 step.  A DFMA whose three operands are
+// different 64-bit registers issues every 3 cycles (0.66 of the pipe), one with
+// two, or a product or a sum, every 2; six of the step's eight instructions have
+// three, so a step takes 22 cycles of a scheduler, 0.727 of the pipe's issue
+// rate.  Two chains with the same coefficients and no tracking reach 0.75
+// (operands reused), with the tracking 0.71, which is what the pair loop runs at.
 #include "lle_device.cuh"
 
 namespace cbf {
@@ -107,14 +113,36 @@ cudaError_t launch_seeds_d(const DevJob& J, double* d_out, cudaStream_t s)
     return cudaGetLastError();
 }
 
-template <class S, bool IC, int PPT, int THREADS, int MINB, int UNR = 2>
+// CAP > 0: at most CAP resident blocks per SM, by asking for shared memory the
+// kernel does not use -- unless CAP + 1 blocks per SM hold the whole grid.
+//
+// Why a cap: a scheduler issues these FP64 chains two warps at a time -- with two
+// chains a thread, 1 to 8 warps per scheduler take 1.29, 1.55, 2.48, 2.88, 3.99,
+// 4.30, -, 5.67 ms on the same per-thread work -- so what counts is that few
+// rounds end on an odd number of warps, not how many are resident: six blocks'
+// worth of points an SM takes 5.27 ms as 5 + 1 and 4.30 ms as 4 + 2, five blocks'
+// worth 4.29 ms as 4 + 1 and 3.99 ms at once.
+template <class S, bool IC, int PPT, int THREADS, int MINB, int UNR = 2, int CAP = 0>
 cudaError_t launch_variant(const DevJob& J, double* d_out, cudaStream_t s)
 {
+    auto kern = lle_kernel<S, IC, PPT, THREADS, MINB, UNR>;
     const long long nq = (J.nPoints + PPT - 1) / PPT;
     const long long blocks = (nq + THREADS - 1) / THREADS;
     const unsigned grid = (unsigned)(blocks < (1ll << 30) ? blocks : (1ll << 30));
     if (grid == 0) return cudaSuccess;
-    lle_kernel<S, IC, PPT, THREADS, MINB, UNR><<<grid, THREADS, 0, s>>>(J, d_out);
+    size_t smem = 0;
+    if constexpr (CAP > 0) {
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (blocks <= (long long)CAP * sms || blocks > (CAP + 1ll) * sms) {
+            smem = (224 / (CAP + 1) + 2) * 1024;  // CAP of these fit an SM's 227 KB, CAP + 1 do not
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    kern<<<grid, THREADS, smem, s>>>(J, d_out);
     note_launch();
     return cudaGetLastError();
 }
@@ -122,7 +150,11 @@ cudaError_t launch_variant(const DevJob& J, double* d_out, cudaStream_t s)
 // The kernel shapes the autotuner chooses from: {points per thread, threads per
 // block, minimum resident blocks per SM (a register cap for the compiler),
 // unrolling of the step loop}.
-//   0: 1 pt, 128 thr, >= 8 blocks/SM  (<= 64 registers, 32 warps/SM), unroll 2  default
+//   0: the default.  Chen and Lorenz in the rescaled step: 1 pt, 128 thr, 90
+//      registers, at most 4 blocks per SM, unroll 8.  The other steps wait for
+//      divisions or for many more operands: where the grid gives an SM more than
+//      4 blocks, as shape 6 (32 warps/SM; 5-D model, 700^2: 27.0 against 28.4 ms),
+//      else as shape 5 (nothing spilled; 64^2: 2.8 against 3.7 ms)
 //   1: 1 pt, 128 thr, no cap, unroll 2
 //   2: 1 pt, 256 thr, >= 4 blocks/SM  (<= 64 registers), unroll 2
 //   3: 2 pt, 128 thr, >= 4 blocks/SM  (<= 128 registers, 4 chains per thread), unroll 2
@@ -130,6 +162,9 @@ cudaError_t launch_variant(const DevJob& J, double* d_out, cudaStream_t s)
 //   5: 1 pt, 128 thr, no cap, unroll 4
 //   6: 1 pt, 128 thr, >= 8 blocks/SM, unroll 4
 //   7: 1 pt, 128 thr, no cap, unroll 8
+// Chen 1024^2, 50 000 transient steps and 100 000 pairs: shapes 1..7 take 173,
+// 181, 178, 178, 172, 180, 170 ms, 64 registers with unroll 2 (the default
+// before) 182, the default now 170 (lle map at full length: 908 -> 848 ms).
 template <class S, bool IC>
 cudaError_t launch_lle_v(const DevJob& J, double* d_out, cudaStream_t s, int variant)
 {
@@ -141,7 +176,14 @@ cudaError_t launch_lle_v(const DevJob& J, double* d_out, cudaStream_t s, int var
     case 5: return launch_variant<S, IC, 1, 128, 1, 4>(J, d_out, s);
     case 6: return launch_variant<S, IC, 1, 128, 8, 4>(J, d_out, s);
     case 7: return launch_variant<S, IC, 1, 128, 1, 8>(J, d_out, s);
-    default: return launch_variant<S, IC, 1, 128, 8>(J, d_out, s);
+    default:
+        if constexpr (S::SCALED) return launch_variant<S, IC, 1, 128, 1, 8, 4>(J, d_out, s);
+        int dev = 0, sms = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        return J.nPoints > 4ll * 128 * sms ? launch_variant<S, IC, 1, 128, 8, 4>(J, d_out, s)
+                                           : launch_variant<S, IC, 1, 128, 1, 4>(J, d_out, s);
     }
 }
 
