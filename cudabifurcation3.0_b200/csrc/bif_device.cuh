@@ -134,7 +134,7 @@ __device__ __forceinline__ bool record_loop(const RecordSpec& R, double (&x)[S::
                 tr.add2(a, p);
             }
             if (!tr.maybe(R.hiT)) {
-                ps.push_block<kRing, WITH_INTERVALS>(up, t, p, ring, pk, iv, R.cap, hook);
+                ps.push_block<kRing, WITH_INTERVALS>(up, t, kRing, p, ring, pk, iv, R.cap, hook);
                 t += kRing;
                 continue;
             }

@@ -211,15 +211,17 @@ cudaError_t launch_lle_seeds(const DevJob& J, double* d_out, cudaStream_t s);
 cudaError_t launch_ls(const DevJob& J, double* d_out, cudaStream_t s);
 cudaError_t launch_ls_seeds(const DevJob& J, double* d_out, cudaStream_t s);
 cudaError_t launch_lle_regime(const DevJob& J, double* d_lle, int* d_class, cudaStream_t s);
-// Points the LLE_REGIME kernel keeps in flight at once on the current device.
-long long lle_regime_resident_points(const DevJob& J);
+// Points of one wave of the surrogate map's recompute rounds on the current device.
+long long lle_regime_round_points(const DevJob& J);
 // The LLE_REGIME kernel over a device point list (J.pointIndex) whose length
 // *nDev (at most maxPoints) a previous kernel wrote, with caller-provided
 // scratch of lle_regime_scratch_bytes(J); no allocation, no host
-// synchronisation: a device-side check sets *err (zero on entry).
+// synchronisation: a device-side check sets *err (zero on entry); *queue is the
+// launch's tile counter.
 size_t lle_regime_scratch_bytes(const DevJob& J);
 cudaError_t launch_lle_regime_list(const DevJob& J, const long long* nDev, long long maxPoints, double* d_lle,
-                                   int* d_cls, double* scratch, size_t scratchBytes, int* err, cudaStream_t s);
+                                   int* d_cls, double* scratch, size_t scratchBytes, int* err,
+                                   unsigned long long* queue, cudaStream_t s);
 
 // KDE/DBSCAN with caller-provided scratch (no allocation): `scratch` holds
 // `scratchBytes` of peak buffers, `err` one int that must be zero on entry.

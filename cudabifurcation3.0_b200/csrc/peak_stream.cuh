@@ -125,18 +125,18 @@ struct PeakStream {
         prev1 = v;
     }
 
-    // K samples at once: the samples of times t+1 .. t+K (prev1 is time t's), all
-    // of them numbers, in ring[32 * 1] .. ring[32 * K] with time t's in ring[0];
-    // bit K-1-i of `up`: sample t+1+i is above its predecessor.  Equal to K calls
+    // m <= K samples at once: the samples of times t+1 .. t+m (prev1 is time t's),
+    // all of them numbers, in ring[32 * 1] .. ring[32 * m] with time t's in ring[0];
+    // bit K-1-i of `up`: sample t+1+i is above its predecessor.  Equal to m calls
     // of push().  A candidate arrival is one that does not rise after one that
     // did.  The SKIP after a peak is implied -- a sample right after a descent
     // cannot be such an arrival -- so only plateaus need the state.
     template <int K, bool WITH_INTERVALS, class Hook>
-    __host__ __device__ __forceinline__ void push_block(unsigned up, int t, double last, const double* ring, double* pk,
-                                               double* iv, int cap, Hook& hook)
+    __host__ __device__ __forceinline__ void push_block(unsigned up, int t, int m, double last, const double* ring,
+                                                        double* pk, double* iv, int cap, Hook& hook)
     {
-        unsigned cand = ((((unsigned)rising << K) | up) >> 1) & ~up & ((1u << K) - 1u);
-        if (mode != 0) cand = plateau<K, WITH_INTERVALS>(mode == 2 ? -1 : 0, cand, t, ring, pk, iv, cap, hook);
+        unsigned cand = after_rise<K>(up) & ~up & arrivals<K>(m);
+        if (mode != 0) cand = plateau<K, WITH_INTERVALS>(mode == 2 ? -1 : 0, cand, t, m, ring, pk, iv, cap, hook);
         while (cand) {
             const int b = highest_bit(cand);
             const int i = K - 1 - b;
@@ -147,11 +147,23 @@ struct PeakStream {
             } else {
                 mode = 1;
                 pval = a;
-                cand = plateau<K, WITH_INTERVALS>(i + 1, cand, t, ring, pk, iv, cap, hook);
+                cand = plateau<K, WITH_INTERVALS>(i + 1, cand, t, m, ring, pk, iv, cap, hook);
             }
         }
-        rising = (int)(up & 1u);
+        rising = (int)((up >> (K - m)) & 1u);
         prev1 = last;
+    }
+
+    // Arrivals whose predecessor rose (bits as in `up`), and the first m arrivals.
+    template <int K>
+    __host__ __device__ __forceinline__ unsigned after_rise(unsigned up) const
+    {
+        return (((unsigned)rising << K) | up) >> 1;
+    }
+    template <int K>
+    __host__ __device__ __forceinline__ static unsigned arrivals(int m)
+    {
+        return ((1u << K) - 1u) & ~((1u << (K - m)) - 1u);
     }
 
 private:
@@ -159,17 +171,17 @@ private:
     // candidates with the arrival after the plateau's end taken out (SKIP).
     // j = -1: the plateau ended at the last arrival before the block.
     template <int K, bool WITH_INTERVALS, class Hook>
-    __host__ __device__ unsigned plateau(int j, unsigned cand, int t, const double* ring, double* pk, double* iv, int cap,
-                                Hook& hook)
+    __host__ __device__ unsigned plateau(int j, unsigned cand, int t, int m, const double* ring, double* pk,
+                                         double* iv, int cap, Hook& hook)
     {
-        for (; mode == 1 && j < K; ++j) {
+        for (; mode == 1 && j < m; ++j) {
             const double v = ring[32 * j + 32];
             if (v == pval) continue;
             if (v < pval) emit<WITH_INTERVALS>(pval, t + j, pk, iv, cap, hook);
             mode = 2;
             break;
         }
-        if (mode == 2 && j + 1 < K) {
+        if (mode == 2 && j + 1 < m) {
             mode = 0;
             cand &= ~(1u << (K - 2 - j));
         }

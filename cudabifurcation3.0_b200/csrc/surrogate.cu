@@ -688,7 +688,7 @@ cbf_status cbf_lle_map_surrogate(const cbf_job* job, const cbf_surrogate_config*
     if (e == cudaSuccess) e = buf.get(kSlotRl, &rl, n);
     if (e == cudaSuccess) e = buf.get(kSlotRc, &rc, n);
     if (e == cudaSuccess) e = buf.get(kSlotSur, &sur, n);
-    if (e == cudaSuccess) e = buf.get(kSlotErr, &rerr, 1);
+    if (e == cudaSuccess) e = buf.get(kSlotErr, &rerr, 64);  // error flag, then the tile counter
     if (e == cudaSuccess) e = buf.get(kSlotScratch, &scr, (long long)(scrBytes / sizeof(double)) + 1);
     if (e != cudaSuccess) return report_cuda_error(e, "recompute buffers");
     if (scrBytes == 0) return report_error(CBF_ERR_INTERNAL, "recompute: no resident LLE_REGIME blocks");
@@ -713,7 +713,7 @@ cbf_status cbf_lle_map_surrogate(const cbf_job* job, const cbf_surrogate_config*
     if (e == cudaSuccess) e = cudaMemsetAsync(rerr, 0, sizeof(int), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return report_cuda_error(e, "recompute list");
-    long long resident = lle_regime_resident_points(dj);
+    long long resident = lle_regime_round_points(dj);
     if (resident < 4096) resident = 4096;
     const long long target = 2 * resident;
     // Rounds with rule points: at most ceil(n0 / (target/4)).  Expansion marks
@@ -748,7 +748,8 @@ cbf_status cbf_lle_map_surrogate(const cbf_job* job, const cbf_surrogate_config*
         copy_rule_kernel<<<gridFor(target), 256, 0, s>>>(rule, fillList, list, stats);
         note_launch(5);
         if ((e = cudaGetLastError()) != cudaSuccess) return report_cuda_error(e, "recompute list");
-        if ((e = launch_lle_regime_list(rj, nSel, n, rl, rc, scr, scrBytes, rerr, s)) != cudaSuccess)
+        if ((e = launch_lle_regime_list(rj, nSel, n, rl, rc, scr, scrBytes, rerr,
+                                        reinterpret_cast<unsigned long long*>(rerr + 32), s)) != cudaSuccess)
             return report_cuda_error(e, "recompute");
         merge_kernel<<<gridFor(n), 256, 0, s>>>(list, nSel, rl, rc, flag, dLle, dCls, src, sur, stats);
         note_launch();

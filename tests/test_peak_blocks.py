@@ -34,7 +34,7 @@ static int run(const std::vector<double>& d, bool blocks, double* pk, double* iv
             unsigned up = 0;
             for (int i = 0; i <= K; ++i) ring[32 * i] = d[t + i];
             for (int i = 0; i < K; ++i) up = (up << 1) | (d[t + i + 1] > d[t + i] ? 1u : 0u);
-            ps.push_block<K, true>(up, t, d[t + K], ring, pk, iv, cap, hook);
+            ps.push_block<K, true>(up, t, K, d[t + K], ring, pk, iv, cap, hook);
             t += K;
         } else {
             ++t;
