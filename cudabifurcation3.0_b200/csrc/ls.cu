@@ -7,8 +7,8 @@
 // -- D+1 independent FP64 dependency chains per thread, where the reference runs
 // them one after the other from shared memory.  Each trajectory stops at its own
 // first divergence-test violation in the interval, as the reference's separate
-// loopCalculateDiscreteModel calls do (unchecked run with the high-word max on
-// the ALU pipe, exact replay only when the threshold's high word is reached).
+// loopCalculateDiscreteModel calls do (unchecked run with a high-word maximum,
+// exact replay only when the threshold's high word is reached).
 // After every interval the deviations are orthonormalised by the reference's
 // classical Gram-Schmidt (projections against the not yet normalised earlier
 // rows, then normalisation; cudaLibrary.cu:913-956) in its operation order, and
@@ -23,13 +23,21 @@ namespace {
 constexpr int kLsThreads = 128;
 
 // loopCalculateDiscreteModel(t[j], values, h, n, 1, 0, maxValue) for M
-// trajectories sharing one parameter set.
+// trajectories sharing one parameter set (M even).  A divergence tracker takes two
+// trajectories of the rescaled step (where a pair may have reached the threshold
+// both are repeated step by step), one of the longer steps, whose repeats cost more.
+//
+// Bound: the FP64 step's register reads (see lle.cu).  Four chains with the same
+// coefficients run at 0.72 of the FP64 pipe from one or two warps per scheduler
+// on (two high-word integer operations per value, the tracking before: 0.66).
 template <class S, int M>
 __device__ __forceinline__ void run_multi(double (&t)[M][S::DIM], const typename S::Coef& c, int n,
                                           const DevJob& J)
 {
+    static_assert(M % 2 == 0, "trajectories are tracked in pairs");
+    constexpr int UNR = S::SCALED ? 4 : 2, PER = S::SCALED ? 2 : 1;
     if (!J.checkDiv) {
-#pragma unroll 2
+#pragma unroll UNR
         for (int i = 0; i < n; ++i) {
 #pragma unroll
             for (int j = 0; j < M; ++j) S::step(t[j], c);
@@ -37,23 +45,21 @@ __device__ __forceinline__ void run_multi(double (&t)[M][S::DIM], const typename
         return;
     }
     double t0[M][S::DIM];
-    unsigned mx[M];
+    HiTrack tr[M / PER];
 #pragma unroll
-    for (int j = 0; j < M; ++j) {
-        copy_state<S::DIM>(t0[j], t[j]);
-        mx[j] = 0;
-    }
-#pragma unroll 2
+    for (int j = 0; j < M; ++j) copy_state<S::DIM>(t0[j], t[j]);
+#pragma unroll
+    for (int j = 0; j < M / PER; ++j) tr[j].init();
+#pragma unroll UNR
     for (int i = 0; i < n; ++i) {
 #pragma unroll
-        for (int j = 0; j < M; ++j) {
-            S::step(t[j], c);
-            mx[j] = max(mx[j], abs_hi(t[j][0]));
-        }
+        for (int j = 0; j < M; ++j) S::step(t[j], c);
+#pragma unroll
+        for (int j = 0; j < M / PER; ++j) tr[j].add2(t[PER * j][0], t[PER * j + PER - 1][0]);
     }
 #pragma unroll
     for (int j = 0; j < M; ++j) {
-        if (mx[j] >= J.divHi) {
+        if (tr[j / PER].maybe(J.divHi)) {
             copy_state<S::DIM>(t[j], t0[j]);
             for (int i = 0; i < n; ++i) {
                 S::step(t[j], c);
@@ -182,8 +188,8 @@ cudaError_t launch_ls(const DevJob& J, double* d_out, cudaStream_t s)
     switch (J.system) {
     case CBF_SYS_MEMRISTIVE5: return launch_s<Memristive5>(J, d_out, s);
     case CBF_SYS_ROSSLER: return launch_s<Rossler>(J, d_out, s);
-    case CBF_SYS_LORENZ: return J.scaledStep ? launch_s<LorenzScaled>(J, d_out, s) : launch_s<Lorenz>(J, d_out, s);
-    case CBF_SYS_CHEN: return J.scaledStep ? launch_s<ChenScaled>(J, d_out, s) : launch_s<Chen>(J, d_out, s);
+    case CBF_SYS_LORENZ: return J.scaledStep ? (J.unitStep ? launch_s<LorenzScaledU>(J, d_out, s) : launch_s<LorenzScaled>(J, d_out, s)) : launch_s<Lorenz>(J, d_out, s);
+    case CBF_SYS_CHEN: return J.scaledStep ? (J.unitStep ? launch_s<ChenScaledU>(J, d_out, s) : launch_s<ChenScaled>(J, d_out, s)) : launch_s<Chen>(J, d_out, s);
     default: return cudaErrorInvalidValue;
     }
 }
