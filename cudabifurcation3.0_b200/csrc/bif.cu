@@ -466,6 +466,32 @@ cudaError_t launch_bif_prealloc(const DevJob& J, void* d_out, double* scratch, s
     }
 }
 
+namespace {
+
+// A warp per row: the row's first min(count, cap) values to packed[offset[row]..].
+__global__ void pack_peaks_kernel(const double* __restrict__ peaks, const int* __restrict__ counts,
+                                  const long long* __restrict__ offset, long long n, int cap,
+                                  double* __restrict__ packed)
+{
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= n) return;
+    const int m = min(max(counts[row], 0), cap);
+    const double* src = peaks + row * cap;
+    double* dst = packed + offset[row];
+    for (int k = threadIdx.x & 31; k < m; k += 32) dst[k] = src[k];
+}
+
+}  // namespace
+
+cudaError_t launch_pack_peaks(const double* peaks, const int* counts, const long long* offset, long long n, int cap,
+                              double* packed, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    pack_peaks_kernel<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(peaks, counts, offset, n, cap, packed);
+    note_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bif(const DevJob& J, void* d_out, int* d_aux, cudaStream_t s)
 {
     switch (J.system) {

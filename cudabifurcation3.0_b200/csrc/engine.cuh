@@ -204,6 +204,10 @@ cudaError_t launch_lle_variant(const DevJob& J, double* d_out, cudaStream_t s, i
 // The shape cbf_run uses for `system` on the current device (capi.cu).
 int lle_variant_for(int system);
 cudaError_t launch_bif(const DevJob& J, void* d_out, int* d_aux, cudaStream_t s);
+// Rows of `cap` peak slots, the first min(counts[p], cap) of row p filled, to
+// packed[offset[p]..].
+cudaError_t launch_pack_peaks(const double* peaks, const int* counts, const long long* offset, long long n, int cap,
+                              double* packed, cudaStream_t s);
 cudaError_t launch_grid_coords(const DevJob& J, double* d_out, cudaStream_t s);
 cudaError_t launch_lle_seeds(const DevJob& J, double* d_out, cudaStream_t s);
 // Lyapunov spectrum: nIC exponents per point (d_out[p*nIC + i]); seed rows
