@@ -183,10 +183,12 @@ __global__ void scatter_kernel(const T* __restrict__ src, const long long* __res
 // step, of which a warp issues 22), so it costs no more when fewer lanes of a
 // warp are in use, and the epilogues of a tile -- serial within a warp -- spread
 // over more warps (at four warps a step takes 90 cycles; with eight, 180).
+// (The 5-D model's step issues for half its latency: two warps per scheduler.)
+template <class S>
 int tile_points(long long n, int sms)
 {
-    const long long t = (n + 16ll * sms - 1) / (16ll * sms);
-    return (int)std::min(32ll, std::max(1ll, t));
+    const long long warps = (S::DIM == 3 ? 16ll : 8ll) * sms;
+    return (int)std::min(32ll, std::max(1ll, (n + warps - 1) / warps));
 }
 
 // Shape of one launch.
@@ -216,7 +218,7 @@ cudaError_t bif_shape(const DevJob& J, int maxTile, bool keys, BifShape* sh)
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, kBifThreads, sh->smem)) != cudaSuccess)
         return e;
     if (perSm < 1) return cudaErrorInvalidConfiguration;
-    sh->tile = std::min(maxTile, tile_points(J.nPoints, sms));
+    sh->tile = std::min(maxTile, tile_points<S>(J.nPoints, sms));
     const long long nTiles = (J.nPoints + sh->tile - 1) / sh->tile;
     sh->blocks = std::min((nTiles + kBifWarps - 1) / kBifWarps, (long long)sms * perSm);
     sh->peakBytes = (size_t)kBifWarps * sh->tile * J.peakCap * sizeof(double) * (task_with_intervals(TASK) ? 2 : 1);
@@ -354,7 +356,7 @@ cudaError_t prealloc_pass(const DevJob& J, void* d_out, double* scratch, size_t 
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const long long lanes = (long long)(peakBytes / perLane);
     BifShape sh;
-    if ((e = bif_shape<S, TASK>(J, tile_points(2 * lanes, sms), false, &sh)) != cudaSuccess) return e;
+    if ((e = bif_shape<S, TASK>(J, tile_points<S>(2 * lanes, sms), false, &sh)) != cudaSuccess) return e;
     sh.blocks = std::min(sh.blocks, (long long)(peakBytes / sh.peakBytes));
     if (sh.blocks < 1) return cudaErrorInvalidValue;
     BifScratch sc{};

@@ -123,7 +123,7 @@ __device__ __forceinline__ bool record_loop(const RecordSpec& R, double (&x)[S::
             unsigned up = 0;
             double p = ps.prev1;
             ring[0] = p;
-#pragma unroll 2
+#pragma unroll (D == 5 ? 1 : 2)
             for (int i = 0; i < kRing; i += 2) {
                 const double a = next();
                 up = __funnelshift_l((unsigned)__double2hiint(p - a), up, 1);
@@ -199,7 +199,7 @@ __device__ int integrate_point(const DevJob& J, long long g, double* pk, double*
         to_stored<S>(st.x, c);
     }
 
-#pragma unroll 4
+#pragma unroll (D == 5 ? 1 : 4)
     for (int i = 0; i < J.nSkip; ++i) S::step(st.x, c);
 
     if constexpr (TASK == CBF_TASK_TRAJECTORY) {

@@ -151,10 +151,11 @@ cudaError_t launch_variant(const DevJob& J, double* d_out, cudaStream_t s)
 // block, minimum resident blocks per SM (a register cap for the compiler),
 // unrolling of the step loop}.
 //   0: the default.  Chen and Lorenz in the rescaled step: 1 pt, 128 thr, 90
-//      registers, at most 4 blocks per SM, unroll 8.  The other steps wait for
-//      divisions or for many more operands: where the grid gives an SM more than
-//      4 blocks, as shape 6 (32 warps/SM; 5-D model, 700^2: 27.0 against 28.4 ms),
-//      else as shape 5 (nothing spilled; 64^2: 2.8 against 3.7 ms)
+//      registers, at most 4 blocks per SM, unroll 8.  The other steps wait for a
+//      division or for many more operands: as shape 5 (nothing spilled; 5-D model,
+//      64^2: 3.1 against 4.8 ms with shape 6, 500^2: 20.5 against 21.7), for 3-D
+//      steps where the grid gives an SM more than 4 blocks as shape 6 (32 warps/SM;
+//      Rossler, 700^2: 8.4 against 8.6 ms)
 //   1: 1 pt, 128 thr, no cap, unroll 2
 //   2: 1 pt, 256 thr, >= 4 blocks/SM  (<= 64 registers), unroll 2
 //   3: 2 pt, 128 thr, >= 4 blocks/SM  (<= 128 registers, 4 chains per thread), unroll 2
@@ -182,7 +183,7 @@ cudaError_t launch_lle_v(const DevJob& J, double* d_out, cudaStream_t s, int var
         cudaError_t e = cudaGetDevice(&dev);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
-        return J.nPoints > 4ll * 128 * sms ? launch_variant<S, IC, 1, 128, 8, 4>(J, d_out, s)
+        return S::DIM == 3 && J.nPoints > 4ll * 128 * sms ? launch_variant<S, IC, 1, 128, 8, 4>(J, d_out, s)
                                            : launch_variant<S, IC, 1, 128, 1, 4>(J, d_out, s);
     }
 }

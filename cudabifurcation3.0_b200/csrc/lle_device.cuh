@@ -27,7 +27,7 @@ __device__ __forceinline__ void run_checked(double (&x)[PPT][S::DIM],
                                             const DevJob& J)
 {
     if (!J.checkDiv) {
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
         for (int i = 0; i < n; ++i) {
 #pragma unroll
             for (int j = 0; j < PPT; ++j) S::step(x[j], c[j]);
@@ -47,7 +47,7 @@ __device__ __forceinline__ void run_checked(double (&x)[PPT][S::DIM],
             tr[j].init();
         }
         // two steps per update of the tracker
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
         for (int i = 0; i + 1 < m; i += 2) {
 #pragma unroll
             for (int j = 0; j < PPT; ++j) {
@@ -90,7 +90,7 @@ __device__ __forceinline__ void run_pair(double (&x)[PPT][S::DIM], double (&y)[P
                                          const typename S::Coef (&c)[PPT], int n, const DevJob& J)
 {
     if (!J.checkDiv) {
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
         for (int i = 0; i < n; ++i) {
 #pragma unroll
             for (int j = 0; j < PPT; ++j) {
@@ -108,7 +108,7 @@ __device__ __forceinline__ void run_pair(double (&x)[PPT][S::DIM], double (&y)[P
         copy_state<S::DIM>(y0[j], y[j]);
         tr[j].init();
     }
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
     for (int i = 0; i < n; ++i) {
 #pragma unroll
         for (int j = 0; j < PPT; ++j) {

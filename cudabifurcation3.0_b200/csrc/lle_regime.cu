@@ -110,7 +110,7 @@ __device__ __forceinline__ void window_loop(const WindowSpec& W, WindowState<S>&
                 unsigned up = 0;
                 double p = ps.prev1;
                 ring[0] = p;
-#pragma unroll 4
+#pragma unroll (D == 5 ? 1 : 4)
                 for (int k = 1; k <= m; ++k) {
                     S::step(x, c);
                     S::step(y, c);
@@ -275,10 +275,10 @@ __device__ __forceinline__ int regime_tile(const DevJob& J, long long g, bool va
 }
 
 // Blocks per SM, as the LLE map kernel: four for the rescaled Chen/Lorenz step (its
-// rounds should end on even counts of warps per scheduler), six for the steps that
-// wait for divisions.
+// rounds should end on even counts of warps per scheduler) and for the 5-D model
+// (110 registers), six for the 3-D steps that wait for a division.
 template <class S>
-constexpr int kRegBlocks = S::SCALED ? 4 : 6;
+constexpr int kRegBlocks = S::SCALED || S::DIM == 5 ? 4 : 6;
 
 // nDev (optional): the job's point count read on the device, in place of
 // J.nPoints (a point list whose length a previous kernel wrote).

@@ -37,7 +37,7 @@ __device__ __forceinline__ void run_multi(double (&t)[M][S::DIM], const typename
     static_assert(M % 2 == 0, "trajectories are tracked in pairs");
     constexpr int UNR = S::SCALED ? 4 : 2, PER = S::SCALED ? 2 : 1;
     if (!J.checkDiv) {
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
         for (int i = 0; i < n; ++i) {
 #pragma unroll
             for (int j = 0; j < M; ++j) S::step(t[j], c);
@@ -50,7 +50,7 @@ __device__ __forceinline__ void run_multi(double (&t)[M][S::DIM], const typename
     for (int j = 0; j < M; ++j) copy_state<S::DIM>(t0[j], t[j]);
 #pragma unroll
     for (int j = 0; j < M / PER; ++j) tr[j].init();
-#pragma unroll UNR
+#pragma unroll (S::DIM == 5 ? 1 : UNR)
     for (int i = 0; i < n; ++i) {
 #pragma unroll
         for (int j = 0; j < M; ++j) S::step(t[j], c);

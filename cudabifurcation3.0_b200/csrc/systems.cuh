@@ -15,13 +15,106 @@
 
 #include <cuda_runtime.h>
 #include <math.h>
+#include <string.h>
 
 namespace cbf {
+
+// ---------------------------------------------------------------------------
+// Divisions of the 5-D model.
+
+__host__ __device__ __forceinline__ unsigned high_word(double v)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2hiint(v);
+#else
+    unsigned long long b;
+    memcpy(&b, &v, sizeof(b));
+    return (unsigned)(b >> 32);
+#endif
+}
+
+__host__ __device__ __forceinline__ unsigned low_word(double v)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2loint(v);
+#else
+    unsigned long long b;
+    memcpy(&b, &v, sizeof(b));
+    return (unsigned)b;
+#endif
+}
+
+__host__ __device__ __forceinline__ double from_words(unsigned hi, unsigned lo)
+{
+#ifdef __CUDA_ARCH__
+    return __hiloint2double((int)hi, (int)lo);
+#else
+    const unsigned long long b = ((unsigned long long)hi << 32) | lo;
+    double v;
+    memcpy(&v, &b, sizeof(v));
+    return v;
+#endif
+}
+
+// Where a value's magnitude lies: 0 for zeros, below kOperandSpan in [2^-200, 2^200),
+// at or above it elsewhere (smaller magnitudes wrap around).
+constexpr unsigned kOperandSpan = 2u * (0x4c700000u - 0x33700000u);
+__host__ __device__ __forceinline__ unsigned operand_place(double v)
+{
+    const unsigned hi = high_word(v), twice = hi + hi;
+    return (twice | low_word(v)) == 0u ? 0u : twice - 2u * 0x33700000u;
+}
+
+// Division by a number b that is the same for all steps of a point, correctly
+// rounded like a / b, for a zero or an a in [2^-200, 2^200) and a b well inside the
+// range.  With y = 1/b rounded, Markstein's theorem (IBM J. Res. Dev. 34, 1990: q
+// within an ulp of a/b, r = a - b q exact, then q + r y rounds to RN(a/b)): the
+// first quotient a y is within 1.5 ulp, one correction brings it within one, the
+// second rounds it correctly.  (The corrections of a zero can lose its sign.)
+struct ConstDivisor {
+    double b, y;
+};
+
+__host__ __device__ __forceinline__ bool divisor_in_range(double b)
+{
+    const double m = fabs(b);
+    return m > 0x1p-300 && m < 0x1p300;
+}
+
+__host__ __device__ __forceinline__ double divide(double a, const ConstDivisor& d)
+{
+    const double q0 = a * d.y;
+    const double q1 = fma(fma(-d.b, q0, a), d.y, q0);
+    const double q2 = fma(fma(-d.b, q1, a), d.y, q1);
+    return from_words((high_word(q2) & 0x7fffffffu) | (high_word(q0) & 0x80000000u), low_word(q2));
+}
+
+// a / b; a zero divided by a number leaves the division's general path, which is
+// several times slower (a fixed point at the origin divides zeros at every step).
+__host__ __device__ __forceinline__ double divide_maybe_zero(double a, double b)
+{
+    const bool zero = a == 0.0 && fabs(b) > 0.0;
+    const double q = (zero ? 1.0 : a) / b;
+    return zero ? from_words((high_word(a) ^ high_word(b)) & 0x80000000u, 0u) : q;
+}
 
 // ---------------------------------------------------------------------------
 // The 5-D memristive model compiled into the reference (cudaLibrary.cu:2-44),
 // restated literally: no explicit FMA, and the FP32 quirks of `float y[5], k`
 // (:19) kept -- k and the explicit-half snapshot are rounded to float.
+//
+// Two of the three divisions have divisors of the parameters alone; those run as
+// above, with one look at both dividends' ranges (5 dependent FP64 operations each
+// where the compiler's division takes about 125 cycles).  LLE of 32^2 points 5.0 ->
+// 3.1 ms, a basin map of 231^2 points, one of them the fixed point at the origin,
+// 16.0 -> 5.9 ms, of 500^2 points 26.2 -> 23.7 ms.  The third divisor is known well
+// before its dividend, but its reciprocal taken ahead the same way made a step
+// longer (32^2 points: 3.7 ms): the compiler's reciprocal is a branch that nothing
+// overlaps.
+// Rounding to float by integer operations on the words instead of the conversions
+// there and back made a step shorter by itself but a full SM's steps longer: five
+// roundings are 30 integer operations at half rate, and the conversions have a
+// pipe of their own.
 struct Memristive5 {
     static constexpr int DIM = 5;
     static constexpr int NV = 8;
@@ -31,6 +124,8 @@ struct Memristive5 {
         double a0, a1, a2, a3, a4, a5, a6;
         double kd;  // (double)(float)(h * a7)
         double h1;  // h * (1 - a7)
+        ConstDivisor d2, d3;  // 1 + h1 * a1, 1 + h1 * a3
+        unsigned span;        // kOperandSpan, or 0 where a divisor is out of range
     };
     __host__ __device__ static Coef prep(const double* a, double h)
     {
@@ -40,11 +135,18 @@ struct Memristive5 {
         float k = (float)(h * a[7]);
         c.kd = (double)k;
         c.h1 = h * (1 - a[7]);
+        c.d2.b = 1 + c.h1 * c.a1;
+        c.d3.b = 1 + c.h1 * c.a3;
+        c.d2.y = 1.0 / c.d2.b;
+        c.d3.y = 1.0 / c.d3.b;
+        c.span = divisor_in_range(c.d2.b) && divisor_in_range(c.d3.b) ? kOperandSpan : 0u;
         return c;
     }
-    __device__ __forceinline__ static void step(double* x, const Coef& c)
+    // LITERAL: the divisions as written (what step() is compared with).
+    template <bool LITERAL>
+    __host__ __device__ __forceinline__ static void evaluate(double* x, const Coef& c)
     {
-        const double k = c.kd;
+        const double k = c.kd, h1 = c.h1;
         x[4] = x[4] + k * (x[0]);
         x[3] = x[3] + k * (-c.a2 * x[1] - c.a3 * x[3]);
         x[2] = x[2] + k * (c.a1 * (x[1] - x[0] - x[2]));
@@ -57,13 +159,24 @@ struct Memristive5 {
         const double y3 = (double)(float)x[3];
         const double y4 = (double)(float)x[4];
 
-        const double h1 = c.h1;
-        x[0] = (y0 + h1 * (c.a0 * x[2])) / (1 + h1 * c.a0 * (c.a4 + c.a5 + c.a6 * fabs(x[4])));
+        const double n0 = y0 + h1 * (c.a0 * x[2]);
+        const double d0 = 1 + h1 * c.a0 * (c.a4 + c.a5 + c.a6 * fabs(x[4]));
+        x[0] = LITERAL ? n0 / d0 : divide_maybe_zero(n0, d0);
         x[1] = y1 + h1 * (-x[2] + x[3]);
-        x[2] = (y2 + h1 * (c.a1 * (x[1] - x[0]))) / (1 + h1 * c.a1);
-        x[3] = (y3 + h1 * (-c.a2 * x[1])) / (1 + h1 * c.a3);
+        const double n2 = y2 + h1 * (c.a1 * (x[1] - x[0]));
+        const double n3 = y3 + h1 * (-c.a2 * x[1]);
+        x[2] = LITERAL ? n2 / c.d2.b : divide(n2, c.d2);
+        x[3] = LITERAL ? n3 / c.d3.b : divide(n3, c.d3);
+        if (!LITERAL) {
+            const unsigned p2 = operand_place(n2), p3 = operand_place(n3);
+            if ((p2 > p3 ? p2 : p3) >= c.span) {
+                x[2] = n2 / c.d2.b;
+                x[3] = n3 / c.d3.b;
+            }
+        }
         x[4] = y4 + h1 * (x[0]);
     }
+    __host__ __device__ __forceinline__ static void step(double* x, const Coef& c) { evaluate<false>(x, c); }
 };
 
 // ---------------------------------------------------------------------------
