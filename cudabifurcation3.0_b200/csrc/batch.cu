@@ -7,7 +7,8 @@
 // kernel compiled with that family's code only (so each gets its tasks'
 // register count and occupancy); with both present the two kernels run
 // concurrently on forked streams:
-//   * every job is cut into tiles of 32 points (one warp: a lane per point);
+//   * every job is cut into tiles of 32 points (one warp: a lane per point; fewer
+//     points in a small batch of peak jobs, whose epilogues run one by one);
 //   * jobs are ordered by estimated cost per point, longest first, and a prefix
 //     table of tile counts maps a global tile number to (job, tile);
 //   * each warp takes the next tile number from a device counter (atomicAdd by
@@ -41,49 +42,64 @@ struct BatchJob {
     int* aux;
 };
 
+// Peak scratch of a launch: 32 lanes of `stride` slots per warp, and the epilogues
+// the warps share (bif_device.cuh).
+struct BatchScratch {
+    double* peaks;
+    double* intervals;
+    int stride;
+    EpilogueShare share;
+};
+
+// What a warp has of its shared memory.
+struct WarpArea {
+    unsigned* L;
+    unsigned* Sb;
+    DbscanSort so;
+};
+
+// The epilogue of point p (n peaks in the given slot) of a KDE or DBSCAN job.
+__device__ __forceinline__ void bif_epilogue(const BatchJob& B, long long p, int n, const BatchScratch& sc,
+                                             long long slot, const WarpArea& wa, int lane, int* err)
+{
+    const double* pk = sc.peaks + slot * sc.stride;
+    int r;
+    if (B.job.task == CBF_TASK_KDE)
+        r = kde_warp<true>(kde_spec(B.job), pk, n, lane, reinterpret_cast<float*>(wa.L), kKdeSortCap);
+    else
+        r = dbscan_warp(dbscan_spec(B.job), pk, sc.intervals + slot * sc.stride, n, lane, wa.L, wa.Sb, err, wa.so);
+    if (lane == 0) ((int*)B.out)[p] = r;
+    __syncwarp();
+}
+
+// Integrates a tile: the emitted peaks of this lane's point.
 template <class S, int TASK>
-__device__ __forceinline__ void bif_tile(const DevJob& J, void* out, int* aux, long long p0, int lane,
-                                         double* slotPk, double* slotIv, int stride, unsigned* L,
-                                         unsigned* Sb, const DbscanSort& so, int* err)
+__device__ __forceinline__ int bif_tile(const DevJob& J, void* out, int* aux, long long p0, int tilePts, int lane,
+                                        const BatchScratch& sc, long long warpId, const WarpArea& wa)
 {
     const long long p = p0 + lane;
-    const bool valid = p < J.nPoints;
-    const long long g = grid_index(J, p);
+    const bool valid = lane < tilePts && p < J.nPoints;
+    const long long g = valid ? grid_index(J, p) : 0;
+    double* ring = ring_column(wa.L, lane);
     if (TASK == CBF_TASK_PEAKS) {
         if (valid) {
             double* pk = (double*)out + p * (long long)J.peakCap;
-            aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, J.peakCap, nullptr, nullptr, ring_column(L, lane));
+            aux[p] = integrate_point<S, TASK>(J, g, pk, nullptr, J.peakCap, nullptr, nullptr, ring);
         }
-        return;
+        return 0;
     }
-    double* myPk = slotPk + (long long)lane * stride;
-    double* myIv = (TASK == CBF_TASK_DBSCAN) ? slotIv + (long long)lane * stride : nullptr;
-    int n = 0;
-    if (valid) n = integrate_point<S, TASK>(J, g, myPk, myIv, J.peakCap, nullptr, nullptr, ring_column(L, lane));
-    __syncwarp();
-    int res = 0;
-    const int live = (int)min((long long)kTile, J.nPoints - p0);
-    for (int j = 0; j < live; ++j) {
-        const int nj = __shfl_sync(kFull, n, j);
-        const double* pk = slotPk + (long long)j * stride;
-        int r;
-        if (TASK == CBF_TASK_KDE)
-            r = kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
-        else
-            r = dbscan_warp(dbscan_spec(J), pk, slotIv + (long long)j * stride, nj, lane, L, Sb, err, so);
-        if (lane == j) res = r;
-    }
-    if (valid) ((int*)out)[p] = res;
-    __syncwarp();
+    const long long slot = warpId * kTile + lane;
+    double* myPk = sc.peaks + slot * sc.stride;
+    double* myIv = (TASK == CBF_TASK_DBSCAN) ? sc.intervals + slot * sc.stride : nullptr;
+    return valid ? integrate_point<S, TASK>(J, g, myPk, myIv, J.peakCap, nullptr, nullptr, ring) : 0;
 }
 
 // FAM: the kernel family -- kFamLle runs LLE jobs only, kFamPeaks the
 // peak-based tasks (PEAKS, KDE, DBSCAN).  Each family is compiled with its own
 // code only, so its register count and occupancy are those of its tasks.
 template <class S, int FAM>
-__device__ __forceinline__ void run_tile(const DevJob& J, void* out, int* aux, long long p0, int lane,
-                                         double* slotPk, double* slotIv, int stride, unsigned* L,
-                                         unsigned* Sb, const DbscanSort& so, int* err)
+__device__ __forceinline__ int run_tile(const DevJob& J, void* out, int* aux, long long p0, int tilePts, int lane,
+                                        const BatchScratch& sc, long long warpId, const WarpArea& wa)
 {
     if constexpr (FAM == kFamLle) {
         const long long p = p0 + lane;
@@ -91,35 +107,29 @@ __device__ __forceinline__ void run_tile(const DevJob& J, void* out, int* aux, l
             const long long g = grid_index(J, p);
             ((double*)out)[p] = J.sweepIC ? lle_point<S, true>(J, g) : lle_point<S, false>(J, g);
         }
-        return;
+        return 0;
     } else {
-    switch (J.task) {
-    case CBF_TASK_KDE:
-        bif_tile<S, CBF_TASK_KDE>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-        break;
-    case CBF_TASK_DBSCAN:
-        bif_tile<S, CBF_TASK_DBSCAN>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-        break;
-    case CBF_TASK_PEAKS:
-        bif_tile<S, CBF_TASK_PEAKS>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-        break;
-    default:
-        break;
-    }
+        switch (J.task) {
+        case CBF_TASK_KDE: return bif_tile<S, CBF_TASK_KDE>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+        case CBF_TASK_DBSCAN: return bif_tile<S, CBF_TASK_DBSCAN>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+        case CBF_TASK_PEAKS: return bif_tile<S, CBF_TASK_PEAKS>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+        default: return 0;
+        }
     }
 }
 
 // WITH_M5: also dispatch the 5-D shipped model.  Its wider state raises the
 // register count of the whole kernel, so batches of 3-D systems use the
 // instantiation without it.
-// Both families are bounded to 6 blocks of 128 threads per SM (80 registers):
-// the occupancy of the autotuned LLE map kernel, and for the peak family 1.5x
-// what its register count would otherwise allow, which is worth the small
-// spill of its epilogue paths (batch64: 43.6 s instead of 49.2 s).
+// Four blocks of 128 threads per SM (128 registers) in both families: the FP64
+// chains issue best from an even number of warps per scheduler (see lle.cu; at six
+// blocks the LLE jobs of a 24-job mix took 30 ms, at four 24).  Peak jobs' epilogues
+// are shared by the warps that have run out of tiles (the same mix's peak jobs: 43
+// -> 35 ms; the two families side by side, two blocks per SM each, were no faster).
 template <int FAM, bool WITH_M5>
-__global__ void __launch_bounds__(kBatchThreads, 6) batch_kernel(
+__global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(
     const BatchJob* __restrict__ jobs, int nJobs, const long long* __restrict__ tileEnd,
-    unsigned long long* counter, double* scrPk, double* scrIv, int stride, int bitWords, int sortCap, int* err)
+    unsigned long long* counter, const BatchScratch sc, int tilePts, int bitWords, int sortCap, int* err)
 {
     extern __shared__ __align__(16) unsigned smem[];
     __shared__ long long sEnd[kMaxBatchJobs];
@@ -129,61 +139,80 @@ __global__ void __launch_bounds__(kBatchThreads, 6) batch_kernel(
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const long long warpId = (long long)blockIdx.x * kBatchWarps + wib;
-    unsigned* L = smem + (size_t)wib * dbscan_warp_words(bitWords, sortCap);
-    unsigned* Sb = L + bitWords;
-    const DbscanSort so = dbscan_sort_area(L, bitWords, sortCap);
-    double* slotPk = scrPk ? scrPk + warpId * kTile * (long long)stride : nullptr;
-    double* slotIv = scrIv ? scrIv + warpId * kTile * (long long)stride : nullptr;
+    WarpArea wa;
+    wa.L = smem + (size_t)wib * dbscan_warp_words(bitWords, sortCap);
+    wa.Sb = wa.L + bitWords;
+    wa.so = dbscan_sort_area(wa.L, bitWords, sortCap);
 
-    for (;;) {
-        unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(counter, 1ull);
-        t = __shfl_sync(kFull, t, 0);
-        if (t >= total) break;
-        int lo = 0, hi = nJobs - 1;  // first job whose tile range ends after t
+    // The job of tile t (the first whose tile range ends after t) and the tile's
+    // first point.
+    auto job_of = [&](unsigned long long t, long long* p0) {
+        int lo = 0, hi = nJobs - 1;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
             if ((unsigned long long)sEnd[mid] > t) hi = mid;
             else lo = mid + 1;
         }
-        const long long firstTile = lo ? sEnd[lo - 1] : 0;
-        const long long p0 = ((long long)t - firstTile) * kTile;
-        void* out = jobs[lo].out;
-        int* aux = jobs[lo].aux;
-        auto go = [&](const DevJob& J) {
+        *p0 = ((long long)t - (lo ? sEnd[lo - 1] : 0)) * tilePts;
+        return lo;
+    };
+
+    for (;;) {
+        unsigned long long t = 0;
+        if constexpr (FAM == kFamPeaks) {
+            t = epilogue_next_tile(sc.share, counter, total, lane);
+        } else {
+            if (lane == 0) t = atomicAdd(counter, 1ull);
+            t = __shfl_sync(kFull, t, 0);
+        }
+        if (t >= total) break;
+        long long p0 = 0;
+        const int k = job_of(t, &p0);
+        void* out = jobs[k].out;
+        int* aux = jobs[k].aux;
+        auto go = [&](const DevJob& J) -> int {
             switch (J.system) {
             case CBF_SYS_MEMRISTIVE5:
-                if (WITH_M5) run_tile<Memristive5, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                break;
-            case CBF_SYS_ROSSLER: run_tile<Rossler, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err); break;
+                if (WITH_M5) return run_tile<Memristive5, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+                return 0;
+            case CBF_SYS_ROSSLER: return run_tile<Rossler, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
             case CBF_SYS_LORENZ:
                 if (J.scaledStep && J.unitStep)  // the map kernels' 8-instruction form
-                    run_tile<LorenzScaledU, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                else if (J.scaledStep)
-                    run_tile<LorenzScaled, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                else
-                    run_tile<Lorenz, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                break;
+                    return run_tile<LorenzScaledU, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+                if (J.scaledStep) return run_tile<LorenzScaled, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+                return run_tile<Lorenz, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
             case CBF_SYS_CHEN:
                 if (J.scaledStep && J.unitStep)  // the map kernels' 8-instruction form
-                    run_tile<ChenScaledU, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                else if (J.scaledStep)
-                    run_tile<ChenScaled, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                else
-                    run_tile<Chen, FAM>(J, out, aux, p0, lane, slotPk, slotIv, stride, L, Sb, so, err);
-                break;
-            default: break;
+                    return run_tile<ChenScaledU, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+                if (J.scaledStep) return run_tile<ChenScaled, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+                return run_tile<Chen, FAM>(J, out, aux, p0, tilePts, lane, sc, warpId, wa);
+            default: return 0;
             }
         };
         // The LLE family reads its descriptor in place (read-only cache); the
         // peak family keeps a copy (fewer registers in its epilogues).
         if constexpr (FAM == kFamLle) {
-            go(jobs[lo].job);
+            go(jobs[k].job);
         } else {
-            const DevJob J = jobs[lo].job;
-            go(J);
+            int n = 0, live = 0;
+            {
+                const DevJob J = jobs[k].job;
+                n = go(J);
+                if (J.task != CBF_TASK_PEAKS) live = (int)min((long long)tilePts, J.nPoints - p0);
+            }
+            __syncwarp();
+            epilogue_publish(sc.share, warpId, lane, n, live, t);
+            epilogue_own(sc.share, warpId, lane, live, [&](int j) {
+                bif_epilogue(jobs[k], p0 + j, sc.share.count[warpId * 32 + j], sc, warpId * kTile + j, wa, lane, err);
+            });
         }
     }
+    if constexpr (FAM == kFamPeaks)
+        epilogue_help(sc.share, warpId, lane, [&](long long from, unsigned long long t, int j) {
+            long long p0 = 0;
+            const int k = job_of(t, &p0);
+            bif_epilogue(jobs[k], p0 + j, sc.share.count[from * 32 + j], sc, from * kTile + j, wa, lane, err);
+        });
 }
 
 // Model steps per point, the batch's cost estimate for ordering.
@@ -195,8 +224,8 @@ double steps_per_point(const DevJob& d)
 
 }  // namespace
 
-using BatchKernel = void (*)(const BatchJob*, int, const long long*, unsigned long long*, double*, double*,
-                            int, int, int, int*);
+using BatchKernel = void (*)(const BatchJob*, int, const long long*, unsigned long long*, const BatchScratch, int, int,
+                            int, int*);
 
 BatchKernel batch_kernel_for(int fam, bool withM5)
 {
@@ -204,9 +233,12 @@ BatchKernel batch_kernel_for(int fam, bool withM5)
     return withM5 ? batch_kernel<kFamPeaks, true> : batch_kernel<kFamPeaks, false>;
 }
 
+// Bytes of the peak family's shared epilogues for a grid of up to `blocks` blocks.
+size_t batch_share_bytes(int blocks) { return epilogue_share_bytes((long long)blocks * kBatchWarps, nullptr); }
+
 cudaError_t batch_launch(const void* jobs, int nJobs, const long long* tileEnd,
-                         unsigned long long* counter, double* scrPk, double* scrIv, int stride,
-                         int bitWords, int* err, int grid, bool withM5, int fam, cudaStream_t s)
+                         unsigned long long* counter, double* scrPk, double* scrIv, int stride, void* share,
+                         int tilePts, int bitWords, int* err, int grid, bool withM5, int fam, cudaStream_t s)
 {
     const int sortCap = bitWords > 0 ? dbscan_sort_cap(bitWords * 32) : 0;
     const size_t smem = (size_t)kBatchWarps * dbscan_warp_words(bitWords, sortCap) * sizeof(unsigned);
@@ -217,8 +249,15 @@ cudaError_t batch_launch(const void* jobs, int nJobs, const long long* tileEnd,
         if (e != cudaSuccess) return e;
     }
     if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
-    kern<<<grid, kBatchThreads, smem, s>>>((const BatchJob*)jobs, nJobs, tileEnd, counter, scrPk, scrIv,
-                                           stride, bitWords, sortCap, err);
+    BatchScratch sc{scrPk, scrIv, stride, EpilogueShare{}};
+    if (fam == kFamPeaks) {
+        size_t zeroed = 0;
+        epilogue_share_bytes((long long)grid * kBatchWarps, &zeroed);
+        sc.share = epilogue_share(share, (long long)grid * kBatchWarps);
+        if ((e = cudaMemsetAsync(share, 0, zeroed, s)) != cudaSuccess) return e;
+    }
+    kern<<<grid, kBatchThreads, smem, s>>>((const BatchJob*)jobs, nJobs, tileEnd, counter, sc, tilePts, bitWords,
+                                           sortCap, err);
     note_launch();
     return cudaGetLastError();
 }
@@ -242,7 +281,7 @@ int batch_tile() { return kTile; }
 int batch_max_jobs() { return kMaxBatchJobs; }
 
 // Host-side plan: order by cost, prefix tile ends, packed device descriptors.
-void batch_plan(const DevJob* jobs, void* const* outs, void* const* auxs, int n,
+void batch_plan(const DevJob* jobs, void* const* outs, void* const* auxs, int n, int tile,
                 std::vector<unsigned char>& packed, std::vector<long long>& tileEnd,
                 std::vector<int>& order)
 {
@@ -262,7 +301,7 @@ void batch_plan(const DevJob* jobs, void* const* outs, void* const* auxs, int n,
         b.out = outs[i];
         b.aux = auxs ? (int*)auxs[i] : nullptr;
         memcpy(packed.data() + (size_t)k * sizeof(BatchJob), &b, sizeof(b));
-        acc += (jobs[i].nPoints + kTile - 1) / kTile;
+        acc += (jobs[i].nPoints + tile - 1) / tile;
         tileEnd[k] = acc;
     }
 }

@@ -11,14 +11,15 @@ namespace cbf {
 constexpr int kFamilies = 2;  // 0: LLE jobs, 1: peak-based jobs (PEAKS, KDE, DBSCAN)
 
 cudaError_t batch_launch(const void* jobs, int nJobs, const long long* tileEnd,
-                         unsigned long long* counter, double* scrPk, double* scrIv, int stride,
-                         int bitWords, int* err, int grid, bool withM5, int fam, cudaStream_t s);
+                         unsigned long long* counter, double* scrPk, double* scrIv, int stride, void* share,
+                         int tilePts, int bitWords, int* err, int grid, bool withM5, int fam, cudaStream_t s);
+size_t batch_share_bytes(int blocks);
 int batch_max_blocks_per_sm(int bitWords, bool withM5, int fam);
 size_t batch_job_bytes();
 int batch_threads();
 int batch_tile();
 int batch_max_jobs();
-void batch_plan(const DevJob* jobs, void* const* outs, void* const* auxs, int n,
+void batch_plan(const DevJob* jobs, void* const* outs, void* const* auxs, int n, int tile,
                 std::vector<unsigned char>& packed, std::vector<long long>& tileEnd,
                 std::vector<int>& order);
 cbf_status run_job_lowered(const DevJob& d, void* d_out, void* d_aux, cudaStream_t s);
@@ -36,6 +37,7 @@ struct BatchFamily {
     bool withM5 = false;      // a job uses the 5-D shipped model
     int maxBlocksPerSm = 0;
     int blocksPerSm = 0;
+    int tile = 32;            // points per tile
     long long points = 0;
 };
 
@@ -50,6 +52,7 @@ struct cbf_batch {
     int* d_err = nullptr;
     double* d_scrPk = nullptr;
     double* d_scrIv = nullptr;
+    void* d_share = nullptr;  // the peak family's shared epilogues (behind the counters)
     int stride = 0;
     int bitWords = 0;
     int sms = 1;
@@ -89,6 +92,7 @@ void release_all(cbf_batch* b)
     b->d_counter = nullptr;
     b->d_scrPk = nullptr;
     b->d_scrIv = nullptr;
+    b->d_share = nullptr;
     b->evFork = b->evJoin = nullptr;
     b->side = nullptr;
 }
@@ -108,7 +112,7 @@ cbf_status upload(cbf_batch* b, int f, const std::vector<DevJob>& jobs, void** d
     std::vector<unsigned char> packed;
     std::vector<long long> tileEnd;
     std::vector<int> order;
-    batch_plan(sub.data(), outs.data(), auxs.data(), (int)sub.size(), packed, tileEnd, order);
+    batch_plan(sub.data(), outs.data(), auxs.data(), (int)sub.size(), F.tile, packed, tileEnd, order);
     cudaError_t e = cudaMalloc(d_jobs, packed.size());
     if (e == cudaSuccess) e = cudaMalloc((void**)d_end, tileEnd.size() * sizeof(long long));
     if (e == cudaSuccess) e = cudaMemcpy(*d_jobs, packed.data(), packed.size(), cudaMemcpyHostToDevice);
@@ -123,7 +127,8 @@ cbf_status launch_family(cbf_batch* b, int f, void* d_jobs, long long* d_end, in
     const BatchFamily& F = b->fam[f];
     const int grid = std::max(1, b->sms * blocksPerSm);
     cudaError_t e = batch_launch(d_jobs, (int)F.jobIdx.size(), d_end, b->d_counter + f, b->d_scrPk, b->d_scrIv,
-                                 b->stride, f == 1 ? b->bitWords : 0, b->d_err, grid, F.withM5, f, s);
+                                 b->stride, b->d_share, F.tile, f == 1 ? b->bitWords : 0, b->d_err, grid, F.withM5, f,
+                                 s);
     if (e != cudaSuccess) return report_cuda_error(e, "batch launch");
     return CBF_OK;
 }
@@ -243,7 +248,17 @@ cbf_status cbf_batch_create(const cbf_job* jobs, int32_t nJobs, void* const* d_o
         if (anyDbscan) b->d_scrIv = b->d_scrPk + blocks * batch_threads() * (size_t)cap;
     }
     for (BatchFamily& F : b->fam) F.blocksPerSm = F.maxBlocksPerSm;
-    e = cudaMalloc((void**)&b->d_counter, 256);
+    size_t share = 0;
+    if (!b->fam[1].jobIdx.empty()) {
+        // Tiles as in the peak maps (bif.cu: tile_points): 32 points, or fewer where
+        // that leaves less than four (with the 5-D model two) warps per scheduler.
+        BatchFamily& F = b->fam[1];
+        const long long warps = (F.withM5 ? 8ll : 16ll) * b->sms;
+        F.tile = (int)std::min((long long)batch_tile(), std::max(1ll, (F.points + warps - 1) / warps));
+        share = batch_share_bytes(b->sms * F.maxBlocksPerSm);
+    }
+    e = cudaMalloc((void**)&b->d_counter, 256 + share);
+    if (e == cudaSuccess) b->d_share = (char*)b->d_counter + 256;
     if (e != cudaSuccess) {
         release_all(b);
         delete b;
@@ -253,7 +268,7 @@ cbf_status cbf_batch_create(const cbf_job* jobs, int32_t nJobs, void* const* d_o
     {  // one-by-one order over all jobs, longest per point first
         std::vector<unsigned char> packed;
         std::vector<long long> tileEnd;
-        batch_plan(b->jobs.data(), b->outs.data(), b->auxs.data(), nJobs, packed, tileEnd, b->order);
+        batch_plan(b->jobs.data(), b->outs.data(), b->auxs.data(), nJobs, batch_tile(), packed, tileEnd, b->order);
     }
     for (int f = 0; f < kFamilies; ++f) {
         if (b->fam[f].jobIdx.empty()) continue;

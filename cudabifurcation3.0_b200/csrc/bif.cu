@@ -79,7 +79,11 @@ struct BifScratch {
     float* keys;
     int keyCap;
     int* err;
+    EpilogueShare share;  // KDE and DBSCAN
 };
+
+// Tasks whose epilogues are shared (OSTROVSKY's need the integrating lane's flags).
+__host__ __device__ constexpr bool task_shares(int task) { return task == CBF_TASK_KDE || task == CBF_TASK_DBSCAN; }
 
 template <class S, int TASK>
 __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(const DevJob J, void* __restrict__ d_out,
@@ -99,10 +103,27 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
     unsigned* Sb = L + bitWords;
     const DbscanSort so = dbscan_sort_area(L, bitWords, sortCap);
     double* ring = ring_column(L, lane);
+    // Point j of the tile that warp `from` integrated.
+    auto epilogue = [&](long long from, long long tile, int j) {
+        const int n = sc.share.count[from * 32 + j];
+        if (n < 0) return;
+        const long long slot = from * tilePts + j;
+        const double* pk = sc.peaks + slot * cap;
+        int r;
+        if constexpr (TASK == CBF_TASK_KDE)
+            r = sc.keyCap > 0 ? kde_warp<false>(kde_spec(J), pk, n, lane, sc.keys + warpId * sc.keyCap, sc.keyCap)
+                              : kde_warp<true>(kde_spec(J), pk, n, lane, reinterpret_cast<float*>(L), kKdeSortCap);
+        else
+            r = dbscan_warp(dbscan_spec(J), pk, sc.intervals + slot * cap, n, lane, L, Sb, sc.err, so);
+        if (lane == 0) ((int*)d_out)[tile * tilePts + j] = r;
+        __syncwarp();
+    };
 
     for (long long next = warpId;; next += nWarps) {
         long long tile = next;
-        if (sc.queue) {
+        if constexpr (task_shares(TASK)) {
+            tile = (long long)epilogue_next_tile(sc.share, sc.queue, (unsigned long long)nTiles, lane);
+        } else if (sc.queue) {
             unsigned long long t = 0;
             if (lane == 0) t = atomicAdd(sc.queue, 1ull);
             tile = (long long)__shfl_sync(kFull, t, 0);
@@ -143,30 +164,25 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
         }
         __syncwarp();
 
-        int res = 0;
         const int live = (int)min((long long)tilePts, J.nPoints - tile * tilePts);
-        for (int j = 0; j < live; ++j) {
-            const int nj = __shfl_sync(kFull, over ? 0 : n, j);
-            const double* pk = sc.peaks + (slot0 + j) * (long long)cap;
-            int r;
-            if (TASK == CBF_TASK_KDE) {
-                r = sc.keyCap > 0
-                        ? kde_warp<false>(kde_spec(J), pk, nj, lane, sc.keys + warpId * sc.keyCap, sc.keyCap)
-                        : kde_warp<true>(kde_spec(J), pk, nj, lane, reinterpret_cast<float*>(L), kKdeSortCap);
-            } else {
-                const double* iv = sc.intervals + (slot0 + j) * (long long)cap;
-                r = dbscan_warp(dbscan_spec(J), pk, iv, nj, lane, L, Sb, sc.err, so);
+        if constexpr (task_shares(TASK)) {
+            epilogue_publish(sc.share, warpId, lane, over ? -1 : n, live, (unsigned long long)tile);
+            epilogue_own(sc.share, warpId, lane, live, [&](int j) { epilogue(warpId, tile, j); });
+        } else {
+            int res = 0;
+            for (int j = 0; j < live; ++j) {
+                const int nj = __shfl_sync(kFull, over ? 0 : n, j);
+                const int r = dbscan_warp(dbscan_spec(J), sc.peaks + (slot0 + j) * (long long)cap,
+                                          sc.intervals + (slot0 + j) * (long long)cap, nj, lane, L, Sb, sc.err, so);
+                if (lane == j) res = r;
             }
-            if (lane == j) res = r;
+            if (valid && !over) ((double*)d_out)[p] = ostrovsky_value(n, div != 0, of, res);
+            __syncwarp();
         }
-        if (valid && !over) {
-            if (TASK == CBF_TASK_OSTROVSKY)
-                ((double*)d_out)[p] = ostrovsky_value(n, div != 0, of, res);
-            else
-                ((int*)d_out)[p] = res;
-        }
-        __syncwarp();
     }
+    if constexpr (task_shares(TASK))
+        epilogue_help(sc.share, warpId, lane,
+                      [&](long long from, unsigned long long tile, int j) { epilogue(from, (long long)tile, j); });
 }
 
 template <class T>
@@ -248,15 +264,18 @@ cudaError_t bif_pass(const DevJob& J, void* d_out, int* d_aux, const Overflow& o
         if ((e = cudaMemGetInfo(&freeB, &totalB)) != cudaSuccess) return e;
         const size_t budget = std::min(freeB / 4, (size_t)8 << 30);
         sh.blocks = std::min(sh.blocks, std::max(1ll, (long long)(budget / sh.blockBytes)));
-        // [error flag, counter | peaks | intervals | keys]
-        if ((e = cudaMallocAsync((void**)&mem, 256 + (size_t)sh.blocks * sh.blockBytes, s)) != cudaSuccess) return e;
+        // [error flag, counter | shared epilogues | peaks | intervals | keys]
+        size_t zeroed = 0;
+        const size_t head = 256 + (epilogue_share_bytes(sh.blocks * kBifWarps, &zeroed) + 255) / 256 * 256;
+        if ((e = cudaMallocAsync((void**)&mem, head + (size_t)sh.blocks * sh.blockBytes, s)) != cudaSuccess) return e;
         sc.err = (int*)mem;
         sc.queue = (unsigned long long*)(mem + 128);
-        sc.peaks = (double*)(mem + 256);
+        sc.share = epilogue_share(mem + 256, sh.blocks * kBifWarps);
+        sc.peaks = (double*)(mem + head);
         if (task_with_intervals(TASK)) sc.intervals = sc.peaks + (size_t)sh.blocks * kBifWarps * sh.tile * J.peakCap;
-        sc.keys = (float*)(mem + 256 + (size_t)sh.blocks * sh.peakBytes);
+        sc.keys = (float*)(mem + head + (size_t)sh.blocks * sh.peakBytes);
         sc.keyCap = sh.keyCap;
-        if ((e = cudaMemsetAsync(mem, 0, 256, s)) != cudaSuccess) {
+        if ((e = cudaMemsetAsync(mem, 0, 256 + zeroed, s)) != cudaSuccess) {
             cudaFreeAsync(mem, s);
             return e;
         }
@@ -339,32 +358,36 @@ cudaError_t launch_bif_s(const DevJob& J, void* d_out, int* d_aux, cudaStream_t 
 }
 
 // One pass of the fused kernel with caller-provided scratch (no allocation);
-// synchronises `s` to read the error flag.  The tile counter takes the first 256
-// bytes; where the scratch holds the lanes of few warps, tiles are smaller
-// (more warps share it).
+// synchronises `s` to read the error flag.  The tile counter and the shared
+// epilogues come first; where the scratch holds the lanes of few warps, tiles are
+// smaller (more warps share it).
 template <class S, int TASK>
 cudaError_t prealloc_pass(const DevJob& J, void* d_out, double* scratch, size_t scratchBytes, int* err,
                           const Overflow& ov, cudaStream_t s)
 {
     if (J.nPoints == 0) return cudaSuccess;
     const size_t perLane = (size_t)J.peakCap * sizeof(double) * (task_with_intervals(TASK) ? 2 : 1);
-    if (scratchBytes < 256 + kBifWarps * perLane) return cudaErrorInvalidValue;
-    const size_t peakBytes = scratchBytes - 256;
     int dev = 0, sms = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const long long lanes = (long long)(peakBytes / perLane);
+    const long long lanes = (long long)(scratchBytes / perLane);
     BifShape sh;
     if ((e = bif_shape<S, TASK>(J, tile_points<S>(2 * lanes, sms), false, &sh)) != cudaSuccess) return e;
-    sh.blocks = std::min(sh.blocks, (long long)(peakBytes / sh.peakBytes));
+    const auto head = [&](long long blocks, size_t* zeroed) {
+        return 256 + (epilogue_share_bytes(blocks * kBifWarps, zeroed) + 255) / 256 * 256;
+    };
+    size_t zeroed = 0;
+    sh.blocks = std::min(sh.blocks, (long long)(scratchBytes / sh.peakBytes));
+    while (sh.blocks > 0 && head(sh.blocks, &zeroed) + (size_t)sh.blocks * sh.peakBytes > scratchBytes) --sh.blocks;
     if (sh.blocks < 1) return cudaErrorInvalidValue;
     BifScratch sc{};
     sc.err = err;
     sc.queue = (unsigned long long*)scratch;
-    sc.peaks = scratch + 32;
+    sc.share = epilogue_share((char*)scratch + 256, sh.blocks * kBifWarps);
+    sc.peaks = (double*)((char*)scratch + head(sh.blocks, &zeroed));
     if (task_with_intervals(TASK)) sc.intervals = sc.peaks + (size_t)sh.blocks * kBifWarps * sh.tile * J.peakCap;
-    if ((e = cudaMemsetAsync(sc.queue, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(scratch, 0, 256 + zeroed, s)) != cudaSuccess) return e;
     bif_kernel<S, TASK><<<(unsigned)sh.blocks, kBifThreads, sh.smem, s>>>(J, d_out, nullptr, sc, sh.bitWords, sh.sortCap,
                                                                           sh.tile, ov);
     note_launch();

@@ -947,5 +947,142 @@ __device__ __noinline__ int dbscan_warp(const DbscanSpec J, const double* pk,
     return cluster - 1;
 }
 
+// ---------------------------------------------------------------------------
+// Epilogues of a tile, shared when the tiles have run out.
+//
+// A tile's epilogues run one after the other in the warp that integrated it, and
+// their cost varies by orders of magnitude (a fixed point's wobble gives a thousand
+// peaks within each other's reach), so maps ended with a few warps at work (Lorenz
+// 1024^2: KDE 188 -> 176 ms, DBSCAN 156 -> 148 ms; 512^2: KDE 49 -> 37 ms).  Every
+// warp therefore publishes its integrated tile, and takes its own points -- and
+// the warps that find no tile left take other warps' points -- by an atomic
+// counter per warp.  A warp's peak slots are reused only with a new tile, which no
+// warp gets once others have found none: nothing a helper reads is overwritten.
+struct EpilogueShare {
+    unsigned* next;             // [warps] points taken of the published tile
+    unsigned long long* info;   // [warps] published tile: payload << 6 | points
+    int* count;                 // [warps * 32] emitted peaks of a point, -1: nothing to do
+    unsigned* busy;             // warps that may hold a tile they have not published
+    int warps;
+};
+
+// Bytes of the share's arrays for `warps` warps; the first `zeroed` of them must
+// be zero on entry.
+__host__ __device__ inline size_t epilogue_share_bytes(long long warps, size_t* zeroed)
+{
+    const size_t z = 256 + (size_t)((warps + 31) / 32 * 32) * (sizeof(unsigned) + sizeof(unsigned long long));
+    if (zeroed) *zeroed = z;
+    return z + (size_t)warps * 32 * sizeof(int);
+}
+
+__host__ __device__ inline EpilogueShare epilogue_share(void* mem, long long warps)
+{
+    const size_t w = (size_t)((warps + 31) / 32 * 32);
+    char* p = static_cast<char*>(mem);
+    EpilogueShare sh;
+    sh.busy = reinterpret_cast<unsigned*>(p);
+    sh.info = reinterpret_cast<unsigned long long*>(p + 256);
+    sh.next = reinterpret_cast<unsigned*>(p + 256 + w * sizeof(unsigned long long));
+    sh.count = reinterpret_cast<int*>(p + 256 + w * (sizeof(unsigned long long) + sizeof(unsigned)));
+    sh.warps = (int)warps;
+    return sh;
+}
+
+// The warp's next tile from the counter `queue`; one of `tiles` or more: none left.
+__device__ __forceinline__ unsigned long long epilogue_next_tile(const EpilogueShare& sh, unsigned long long* queue,
+                                                                 unsigned long long tiles, int lane)
+{
+    unsigned long long t = 0;
+    if (lane == 0) {
+        atomicAdd(sh.busy, 1u);  // before the tile is taken: helpers that see no busy warp miss none
+        __threadfence();
+        t = atomicAdd(queue, 1ull);
+        if (t >= tiles) atomicSub(sh.busy, 1u);
+    }
+    return __shfl_sync(kFull, t, 0);
+}
+
+// This warp's integrated tile: `n` per lane, `payload` names the tile.
+__device__ __forceinline__ void epilogue_publish(const EpilogueShare& sh, long long warp, int lane, int n, int live,
+                                                 unsigned long long payload)
+{
+    sh.count[warp * 32 + lane] = n;
+    __threadfence();  // peaks and counts before the tile
+    __syncwarp();
+    if (lane == 0) {
+        *(volatile unsigned long long*)(sh.info + warp) = payload << 6 | (unsigned)live;
+        __threadfence();
+        atomicExch(sh.next + warp, 0u);
+        __threadfence();
+        atomicSub(sh.busy, 1u);
+    }
+}
+
+// The tile's points by the warp itself: item(j) for every point no helper took.
+// The next point is taken while one is worked on.
+template <class Item>
+__device__ __forceinline__ void epilogue_own(const EpilogueShare& sh, long long warp, int lane, int live, Item item)
+{
+    unsigned j = 0;
+    if (lane == 0) j = atomicAdd(sh.next + warp, 1u);
+    j = __shfl_sync(kFull, j, 0);
+    while (j < (unsigned)live) {
+        unsigned after = 0;
+        if (lane == 0) after = atomicAdd(sh.next + warp, 1u);
+        item((int)j);
+        j = __shfl_sync(kFull, after, 0);
+    }
+    __syncwarp();
+}
+
+// No tile is left: other warps' points until no warp holds a tile that it has not
+// published.  item(warp, payload, j).  The wait for warps that still integrate ends
+// by itself (they are running and need nothing from this one) and after kHelpPolls
+// looks in any case; a helper that leaves early leaves the points to their own warp.
+constexpr int kHelpPolls = 1 << 16;
+template <class Item>
+__device__ __forceinline__ void epilogue_help(const EpilogueShare& sh, long long warp, int lane, Item item)
+{
+    for (int poll = 0; poll < kHelpPolls; ++poll) {
+        unsigned all = 0;
+        if (lane == 0) {
+            all = *(volatile unsigned*)sh.busy == 0u;
+            __threadfence();
+        }
+        all = __shfl_sync(kFull, all, 0);  // read before the look: nothing appears after it
+        bool found = false;
+        for (int base = 0; base < sh.warps; base += 32) {
+            // starts at the warp's own place, so that helpers spread
+            long long v = warp / 32 * 32 + base + lane;
+            if (v >= (sh.warps + 31) / 32 * 32) v -= (sh.warps + 31) / 32 * 32;
+            const bool some = v < sh.warps && *(volatile unsigned*)(sh.next + v) <
+                                                  (unsigned)(*(volatile unsigned long long*)(sh.info + v) & 63u);
+            unsigned mask = __ballot_sync(kFull, some);
+            while (mask) {
+                const int src = __ffs(mask) - 1;
+                mask &= mask - 1;
+                const long long from = __shfl_sync(kFull, v, src);
+                for (;;) {
+                    unsigned j = 0;
+                    unsigned long long info = 0;
+                    if (lane == 0) {
+                        j = atomicAdd(sh.next + from, 1u);
+                        __threadfence();
+                        info = *(volatile unsigned long long*)(sh.info + from);
+                    }
+                    j = __shfl_sync(kFull, j, 0);
+                    info = __shfl_sync(kFull, info, 0);
+                    if (j >= (unsigned)(info & 63u)) break;
+                    __threadfence();  // the tile before its counts and peaks
+                    item(from, info >> 6, (int)j);
+                    found = true;
+                }
+            }
+        }
+        if (all && !found) return;
+        if (!found) __nanosleep(8000);
+    }
+}
+
 }  // namespace
 }  // namespace cbf

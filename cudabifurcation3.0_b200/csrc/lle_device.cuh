@@ -134,6 +134,10 @@ __device__ __forceinline__ void run_pair(double (&x)[PPT][S::DIM], double (&y)[P
     }
 }
 
+// Unrolling of the step loops of one point, as the default LLE shape.
+template <class S>
+constexpr int kPointUnroll = S::SCALED ? 8 : 2;
+
 // One point of LLEKernelCUDA / LLEKernelICCUDA (cudaLibrary.cu:666-908).
 template <class S, bool IC>
 __device__ __forceinline__ double lle_point(const DevJob& J, long long g)
@@ -147,14 +151,14 @@ __device__ __forceinline__ double lle_point(const DevJob& J, long long g)
         c[0] = S::prep(v, J.h);
         to_stored<S>(x[0], c[0]);
     }
-    run_checked<S, 1>(x, c, J.nSkip, J);
+    run_checked<S, 1, kPointUnroll<S>>(x, c, J.nSkip, J);
     double z[D];
     lle_seed<D, IC>(g, J.seedChunk, z);
 #pragma unroll
     for (int i = 0; i < D; ++i) y[0][i] = stored_comp<S>(z[i] * J.lleEps, i, c[0]) + x[0][i];
     double result = 0;
     for (int b = 0; b < J.nRecord; ++b) {
-        run_pair<S, 1>(x, y, c, J.nNT, J);
+        run_pair<S, 1, kPointUnroll<S>>(x, y, c, J.nNT, J);
         double t = 0;
 #pragma unroll
         for (int l = 0; l < D; ++l) {

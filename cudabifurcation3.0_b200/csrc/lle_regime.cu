@@ -198,7 +198,7 @@ __device__ double lle_regime_point(const DevJob& J, long long g, double* ring, d
                                    int* nOut, double* amp)
 {
     constexpr int D = S::DIM;
-    constexpr int UNR = S::SCALED ? 8 : 2;
+    constexpr int UNR = kPointUnroll<S>;
     double x[1][D], y[1][D];
     typename S::Coef c[1];
     {
