@@ -11,14 +11,12 @@
 //
 // Output 0 is the (normalised) LLE, outputs 1..16 the logits of the 16-way
 // peak-count regime class.  Parameters live as FP32 masters (Adam state next to
-// them) plus BF16 copies that feed the tensor cores.  Every matrix product --
-// forward, input gradients, weight gradients, the prediction of explicit
-// feature rows -- runs on the 5th-generation tensor cores through one kernel
-// (mlp_gemm_tc.cuh: TMA-staged operands, tcgen05.mma into tensor memory, fused
-// epilogues); prediction over a whole grid runs as one fused tcgen05 kernel
-// (mlp_tc.cuh).  A training step (minibatch gather, 4 forward products, loss,
-// 7 backward products with their split-K and bias reductions, Adam) is captured
-// once as a CUDA graph and replayed.
+// them) plus BF16 copies that feed the tensor cores.  A training step is three
+// kernels, captured once as a CUDA graph and replayed: minibatch, forward, loss and
+// input gradients as one fused tcgen05 kernel, the weight gradients as one launch of
+// split-K products, and their sums, the bias sums and Adam (mlp_step.cuh).
+// Prediction over a whole grid is one fused tcgen05 kernel (mlp_tc.cuh); explicit
+// feature rows run product by product (mlp_gemm_tc.cuh).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -46,13 +44,13 @@ constexpr long long kW3 = kB2 + kHid, kB3 = kW3 + kHid * kHid;
 constexpr long long kW4 = kB3 + kHid, kB4 = kW4 + kOut * kHid;
 constexpr long long kNumParams = kB4 + kOut;
 
-// Tensor-core operand copies of the weights: seven 256 x 256 BF16 slots (row
-// pitch 256), zero outside the weights: W1 (256 x 128), W2, W3,
-// W4 (17 x 256, rows padded), W2^T, W3^T, W4^T (256 x 17, K padded to 32).
+// Row-major copies of the weights for the products of explicit feature rows: four
+// 256 x 256 BF16 slots (row pitch 256), zero outside the weights: W1 (256 x 128),
+// W2, W3, W4 (17 x 256, rows padded).
 constexpr long long kSlot = (long long)kHid * kHid;
-enum { kSlotW1 = 0, kSlotW2, kSlotW3, kSlotW4, kSlotW2T, kSlotW3T, kSlotW4T, kNumSlots };
+enum { kSlotW1 = 0, kSlotW2, kSlotW3, kSlotW4, kNumSlots };
 constexpr int kXPitch = kIn;   // BF16 first-layer input rows
-constexpr int kDOutPitch = 32;  // BF16 output-gradient rows: 17 values padded to K = 32
+constexpr int kDOutPitch = 32;  // output gradients as an operand: 17 values padded to K = 32
 constexpr int kDOutTRows = 128; // rows of dOut^T (17 used): one full 128-row operand tile
 
 // SiLU z * sigmoid(z) and its derivative.  The sigmoid's quotient uses the
@@ -120,19 +118,6 @@ __device__ __forceinline__ float silu_grad(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
-// C[m*c_m + n*c_n] = sum over z of ws[z][m*N + n], slices added in order.
-__global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int M, int N,
-                                     float* __restrict__ C, long long c_m, long long c_n)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long MN = (long long)M * N;
-    if (i >= MN) return;
-    float acc = 0.f;
-    for (int z = 0; z < splits; ++z) acc += ws[z * MN + i];
-    const long long m = i / N, n = i % N;
-    C[m * c_m + n * c_n] = acc;
-}
-
 // ---- element-wise kernels -------------------------------------------------
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z)
@@ -143,11 +128,14 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z)
     return z ^ (z >> 31);
 }
 
-// Encoded BF16 row r (x: its raw features) into xb (pitch kIn) and, if xT is
-// given, column r of xT (pitch ldT).
-__device__ __forceinline__ void put_encoded_row(const float (&x)[kRaw], long long r, float fs,
-                                                bf16* __restrict__ xb, bf16* __restrict__ xT, long long ldT)
+// Encoded BF16 rows of n raw feature rows X [n x 4].
+__global__ void encode_rows_kernel(const float* __restrict__ X, long long n, float fs, bf16* __restrict__ xb)
 {
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    float x[kRaw];
+#pragma unroll
+    for (int f = 0; f < kRaw; ++f) x[f] = X[r * kRaw + f];
 #pragma unroll 1
     for (int j = 0; j < kIn / 8; ++j) {
         float e[8];
@@ -155,189 +143,8 @@ __device__ __forceinline__ void put_encoded_row(const float (&x)[kRaw], long lon
         reinterpret_cast<uint4*>(xb + r * kXPitch)[j] =
             make_uint4(pack_bf16x2(e[0], e[1]), pack_bf16x2(e[2], e[3]), pack_bf16x2(e[4], e[5]),
                        pack_bf16x2(e[6], e[7]));
-        if (xT) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) xT[(8 * j + i) * ldT + r] = __float2bfloat16_rn(e[i]);
-        }
     }
 }
-
-// Minibatch of B rows drawn uniformly (with replacement) from N, keyed by the
-// device step counter so a replayed graph draws a new batch every step.  The
-// encoded BF16 rows go to xb and, transposed, to xT (row f = input f, pitch
-// ldT) for the first layer's weight gradient.
-__global__ void gather_kernel(const float* __restrict__ X, const float* __restrict__ ylle,
-                              const int* __restrict__ ycls, long long N, int B,
-                              const unsigned long long* step, unsigned long long seed, float fs,
-                              bf16* __restrict__ xb, bf16* __restrict__ xT, long long ldT, float* __restrict__ bl,
-                              int* __restrict__ bc)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B) return;
-    const unsigned long long h = mix64(seed ^ mix64(*step * 0x100000001B3ull + (unsigned long long)r));
-    const long long i = (long long)(h % (unsigned long long)N);
-    float x[kRaw];
-#pragma unroll
-    for (int f = 0; f < kRaw; ++f) x[f] = X[i * kRaw + f];
-    put_encoded_row(x, r, fs, xb, xT, ldT);
-    bl[r] = ylle[i];
-    bc[r] = ycls[i];
-}
-
-// Encoded rows of n raw feature rows X [n x 4] (rows n <= r < rows: zeros).
-__global__ void encode_rows_kernel(const float* __restrict__ X, long long n, long long rows, float fs,
-                                   bf16* __restrict__ xb, bf16* __restrict__ xT, long long ldT)
-{
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    if (r < n) {
-        float x[kRaw];
-#pragma unroll
-        for (int f = 0; f < kRaw; ++f) x[f] = X[r * kRaw + f];
-        put_encoded_row(x, r, fs, xb, xT, ldT);
-    } else {
-        const bf16 zero = __float2bfloat16_rn(0.0f);
-        for (int f = 0; f < kIn; ++f) {
-            xb[r * kXPitch + f] = zero;
-            if (xT) xT[f * ldT + r] = zero;
-        }
-    }
-}
-
-// Loss: mean squared error on output 0 (normalised LLE) + cross-entropy of
-// outputs 1..16; writes dLoss/dOut in FP32 (dOut, pitch 17, for the bias
-// gradient), in BF16 (dOutB, pitch 32, columns 17..31 zero) and transposed in
-// BF16 (dOutT, pitch ldT) for the products, and accumulates the loss.  Rows
-// n <= r < rows (the rest of the last 128-row tile) write zero gradients.
-__global__ void loss_kernel(const float* __restrict__ out, const float* __restrict__ yl,
-                            const int* __restrict__ yc, int n, int rows, float wLle, float* __restrict__ dOut,
-                            bf16* __restrict__ dOutB, bf16* __restrict__ dOutT, long long ldT,
-                            float* __restrict__ lossAcc)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const bf16 zero = __float2bfloat16_rn(0.0f);
-    if (r >= n) {
-        for (int c = 0; c < kDOutPitch; ++c) dOutB[(long long)r * kDOutPitch + c] = zero;
-        for (int c = 0; c < kOut; ++c) dOutT[c * ldT + r] = zero;
-        return;
-    }
-    const float* o = out + (long long)r * kOut;
-    float d[kOut];
-    const float invB = 1.0f / (float)n;
-    const float e = o[0] - yl[r];
-    d[0] = 2.0f * wLle * e * invB;
-    float mx = o[1];
-    for (int c = 1; c < kClasses; ++c) mx = fmaxf(mx, o[1 + c]);
-    float sum = 0.f;
-    for (int c = 0; c < kClasses; ++c) sum += __expf(o[1 + c] - mx);
-    const int t = yc[r];
-    float lossCe = 0.f;
-    for (int c = 0; c < kClasses; ++c) {
-        const float p = __expf(o[1 + c] - mx) / sum;
-        d[1 + c] = (p - (c == t ? 1.0f : 0.0f)) * invB;
-        if (c == t) lossCe = -logf(fmaxf(p, 1e-30f));
-    }
-    for (int c = 0; c < kOut; ++c) {
-        const bf16 v = __float2bfloat16_rn(d[c]);
-        dOut[(long long)r * kOut + c] = d[c];
-        dOutB[(long long)r * kDOutPitch + c] = v;
-        dOutT[c * ldT + r] = v;
-    }
-    for (int c = kOut; c < kDOutPitch; ++c) dOutB[(long long)r * kDOutPitch + c] = zero;
-    atomicAdd(lossAcc, (wLle * e * e + lossCe) * invB);
-}
-
-// db[n] = sum over rows of G[m*ld + n]: a 32x32 block per 32 columns, thread
-// row ty sums rows ty, ty+32, ..., then the 32 partials are added in order.
-__global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ G, int M, int N, long long ld,
-                                                     float* __restrict__ db)
-{
-    __shared__ float part[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int n = blockIdx.x * 32 + tx;
-    float s = 0.f;
-    if (n < N)
-        for (int m = ty; m < M; m += 32) s += G[m * ld + n];
-    part[ty][tx] = s;
-    __syncthreads();
-    if (ty == 0 && n < N) {
-        float t = 0.f;
-        for (int r = 0; r < 32; ++r) t += part[r][tx];
-        db[n] = t;
-    }
-}
-
-cudaError_t colsum(const float* G, int M, int N, long long ld, float* db, cudaStream_t s)
-{
-    colsum_kernel<<<(N + 31) / 32, 1024, 0, s>>>(G, M, N, ld, db);
-    note_launch();
-    return cudaGetLastError();
-}
-
-// BF16 weight w = parameter i into its tensor-core operand slots (and, for W2,
-// W3 and W4, the transposed slot).
-__device__ __forceinline__ void put_weight(bf16* __restrict__ tw, long long i, bf16 w)
-{
-    if (i < kB1) {
-        tw[kSlotW1 * kSlot + (i / kIn) * kHid + i % kIn] = w;
-    } else if (i >= kW2 && i < kB2) {
-        const long long j = i - kW2;
-        tw[kSlotW2 * kSlot + j] = w;
-        tw[kSlotW2T * kSlot + (j % kHid) * kHid + j / kHid] = w;
-    } else if (i >= kW3 && i < kB3) {
-        const long long j = i - kW3;
-        tw[kSlotW3 * kSlot + j] = w;
-        tw[kSlotW3T * kSlot + (j % kHid) * kHid + j / kHid] = w;
-    } else if (i >= kW4 && i < kB4) {
-        const long long j = i - kW4;
-        tw[kSlotW4 * kSlot + j] = w;
-        tw[kSlotW4T * kSlot + (j % kHid) * kHid + j / kHid] = w;
-    }
-}
-
-// Adam on the flat FP32 parameters; refreshes the BF16 weight copies (flat and
-// tensor-core operand slots).
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ gr, float* __restrict__ m1,
-                            float* __restrict__ m2, bf16* __restrict__ pb, bf16* __restrict__ tw, long long n,
-                            float lr0, int horizon, float b1, float b2, float eps, const unsigned long long* step)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const float t = (float)(*step + 1);
-    // cosine decay from lr0 to lr0/20 over `horizon` steps (0: constant)
-    float lr = lr0;
-    if (horizon > 0) {
-        const float u = fminf((float)*step / (float)horizon, 1.0f);
-        lr = lr0 * (0.05f + 0.95f * 0.5f * (1.0f + cospif(u)));
-    }
-    if (i < n) {
-        const float gi = gr[i];
-        const float a = b1 * m1[i] + (1.f - b1) * gi;
-        const float v = b2 * m2[i] + (1.f - b2) * gi * gi;
-        m1[i] = a;
-        m2[i] = v;
-        const float ah = a / (1.f - powf(b1, t));
-        const float vh = v / (1.f - powf(b2, t));
-        const float w = p[i] - lr * ah / (sqrtf(vh) + eps);
-        p[i] = w;
-        const bf16 wb = __float2bfloat16_rn(w);
-        pb[i] = wb;
-        put_weight(tw, i, wb);
-    }
-}
-
-// BF16 copies (flat and operand slots) of the FP32 parameters.
-__global__ void expand_params_kernel(const float* __restrict__ p, bf16* __restrict__ pb, bf16* __restrict__ tw,
-                                     long long n)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const bf16 wb = __float2bfloat16_rn(p[i]);
-    pb[i] = wb;
-    put_weight(tw, i, wb);
-}
-
-__global__ void bump_kernel(unsigned long long* step) { *step += 1; }
 
 // Prediction head: LLE (de-normalised), argmax class, softmax confidence.
 __global__ void head_kernel(const float* __restrict__ out, long long n, float lleMean, float lleStd,
@@ -385,6 +192,45 @@ __global__ void features_kernel(const FeatureSpec f, const long long* __restrict
 #include "mlp_tc.cuh"
 #include "mlp_gemm_tc.cuh"
 
+__device__ __forceinline__ void put_weight(bf16* __restrict__ tw, unsigned char* __restrict__ wp, long long i, bf16 w);
+
+#include "mlp_step.cuh"
+
+// BF16 weight w = parameter i into its row-major slot (tw) and the operand layouts
+// (wp; W2, W3 and W4 transposed too).  Biases have no copy.
+__device__ __forceinline__ void put_weight(bf16* __restrict__ tw, unsigned char* __restrict__ wp, long long i, bf16 w)
+{
+    const auto pack = [&](uint32_t base, int R, int r, int k) { *reinterpret_cast<bf16*>(wp + base + tc_off(R, r, k)) = w; };
+    if (i < kB1) {
+        const int r = (int)(i / kIn), k = (int)(i % kIn);
+        tw[kSlotW1 * kSlot + r * kHid + k] = w;
+        pack(kPkW1, kHid, r, k);
+    } else if (i >= kW2 && i < kB2) {
+        const int r = (int)((i - kW2) / kHid), k = (int)((i - kW2) % kHid);
+        tw[kSlotW2 * kSlot + (i - kW2)] = w;
+        pack(kPkW2, kHid, r, k);
+        pack(kPkW2T, kHid, k, r);
+    } else if (i >= kW3 && i < kB3) {
+        const int r = (int)((i - kW3) / kHid), k = (int)((i - kW3) % kHid);
+        tw[kSlotW3 * kSlot + (i - kW3)] = w;
+        pack(kPkW3, kHid, r, k);
+        pack(kPkW3T, kHid, k, r);
+    } else if (i >= kW4 && i < kB4) {
+        const int r = (int)((i - kW4) / kHid), k = (int)((i - kW4) % kHid);
+        tw[kSlotW4 * kSlot + (i - kW4)] = w;
+        pack(kPkW4, kTcN4, r, k);
+        pack(kPkW4T, kHid, k, r);
+    }
+}
+
+// BF16 copies of the FP32 parameters.
+__global__ void expand_params_kernel(const float* __restrict__ p, bf16* __restrict__ tw, unsigned char* __restrict__ wp,
+                                     long long n)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) put_weight(tw, wp, i, __float2bfloat16_rn(p[i]));
+}
+
 template <class F>
 cudaError_t launch1d(long long n, cudaStream_t s, F f)
 {
@@ -402,12 +248,10 @@ cudaError_t launch1d(long long n, cudaStream_t s, F f)
 
 // Tensor maps of every operand the products read (fixed buffers, built once).
 struct TcMaps {
-    // A operands (128-row tiles): the training batch ...
-    CUtensorMap aX, aH1, aH2, aH3, aDOut, aDZ3, aDZ2, aDOutT, aDZ3T, aDZ2T, aDZ1T;
-    // ... and the prediction workspace
-    CUtensorMap pX, pH1, pH2, pH3;
-    // B operands: weights, transposed weights, transposed activations
-    CUtensorMap bW1, bW2, bW3, bW4, bW4T, bW3T, bW2T, bH3T, bH2T, bH1T, bXT;
+    // weight gradients: A operands dOut^T, dZ^T (128-row tiles), B operands H^T, X^T
+    CUtensorMap aDOutT, aDZ3T, aDZ2T, aDZ1T, bH3T, bH2T, bH1T, bXT;
+    // explicit feature rows: A operands (the prediction workspace), B operands W
+    CUtensorMap pX, pH1, pH2, pH3, bW1, bW2, bW3, bW4;
 };
 
 struct Mlp {
@@ -419,43 +263,38 @@ struct Mlp {
     float* grads = nullptr;
     float* m1 = nullptr;
     float* m2 = nullptr;
-    bf16* pb = nullptr;       // BF16 copies, flat layout (packed for the grid prediction)
-    bf16* tw = nullptr;       // BF16 copies in the tensor-core operand slots
-    // batch buffers (row-major; "T": transposed, pitch Ba)
-    bf16 *xb = nullptr, *xT = nullptr;
-    float* xraw = nullptr;     // raw feature rows of cbf_mlp_forward_backward
+    bf16* tw = nullptr;       // row-major BF16 weights (products of explicit rows)
+    unsigned char* wp = nullptr;  // BF16 weights in the shared-memory operand layout (kPkBytes)
+    // batch buffers ("T": transposed, pitch Ba)
+    float* xraw = nullptr;     // raw feature rows and labels of cbf_mlp_forward_backward
     float* yl = nullptr;
     int* yc = nullptr;
-    float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr;
-    bf16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;
+    bf16* xT = nullptr;
+    float* z = nullptr;        // pre-activations, in the step kernel's own order
     bf16 *h1T = nullptr, *h2T = nullptr, *h3T = nullptr;
     float* out = nullptr;
-    float* dOut = nullptr;
-    bf16 *dOutB = nullptr, *dOutT = nullptr;
-    float* dzf = nullptr;     // FP32 dZ3, dZ2, dZ1 (for the bias gradients), Ba x 256 each
-    bf16 *dz3 = nullptr, *dz2 = nullptr;
-    bf16 *dz3T = nullptr, *dz2T = nullptr, *dz1T = nullptr;
+    float* gradT = nullptr;    // FP32 dOut, dZ3, dZ2, dZ1 for the bias gradients
+    bf16 *dOutT = nullptr, *dz3T = nullptr, *dz2T = nullptr, *dz1T = nullptr;
     float* loss = nullptr;
     float* ws = nullptr;      // split-K partials, one region per weight gradient
-    int* gemmErr = nullptr;   // set by a product whose bounded wait ran out
-    cudaStream_t side = nullptr;  // weight gradients beside the input-gradient chain
-    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    int* gemmErr = nullptr;   // set by a kernel whose bounded wait ran out
     unsigned long long* step = nullptr;
+    unsigned* finished = nullptr;  // blocks of the Adam kernel done
     TcMaps* maps = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     const float* gX = nullptr;  // training set the graph was captured for
+    const float* gYl = nullptr;
+    const int* gYc = nullptr;
     long long gN = 0;
     float gLr = 0.f;
     int gHorizon = 0;
     float gW = 0.f;
     float gScale = 0.f;
     unsigned long long gSeed = 0;
-    // prediction workspace (rows per chunk = kPredRows), no pre-activations
+    // prediction workspace (rows per chunk = kPredRows)
     bf16 *pxb = nullptr, *ph1 = nullptr, *ph2 = nullptr, *ph3 = nullptr;
     float* pout = nullptr;
-    // grid prediction on tcgen05: weights in the shared-memory operand layout
-    unsigned char* wpack = nullptr;
     int* tcErr = nullptr;
 };
 
@@ -488,51 +327,26 @@ cudaError_t pred_workspace(Mlp* m)
     return e;
 }
 
-// Buffers of one forward pass: A-operand maps of the input and hidden
-// activations, and where the pass writes (Z and the transposes may be null).
-struct FwdBufs {
-    const CUtensorMap *aX, *aH1, *aH2, *aH3;
-    float *z1, *z2, *z3;
-    bf16 *h1, *h2, *h3;
-    bf16 *h1T, *h2T, *h3T;
-    long long ldT;
-    float* out;
-};
-
-FwdBufs train_bufs(Mlp& m)
-{
-    const TcMaps& mp = *m.maps;
-    return FwdBufs{&mp.aX, &mp.aH1, &mp.aH2, &mp.aH3, m.z1, m.z2, m.z3, m.h1, m.h2, m.h3,
-                   m.h1T, m.h2T, m.h3T, m.Ba, m.out};
-}
-
-FwdBufs pred_bufs(Mlp& m)
-{
-    const TcMaps& mp = *m.maps;
-    return FwdBufs{&mp.pX, &mp.pH1, &mp.pH2, &mp.pH3, nullptr, nullptr, nullptr, m.ph1, m.ph2, m.ph3,
-                   nullptr, nullptr, nullptr, 0, m.pout};
-}
-
-// Forward on n rows whose BF16 inputs are in the buffer behind f.aX.
-cudaError_t forward(Mlp& m, int n, const FwdBufs& f, cudaStream_t s)
+// Forward on n rows whose BF16 inputs are in the prediction workspace.
+cudaError_t forward(Mlp& m, int n, cudaStream_t s)
 {
     const TcMaps& mp = *m.maps;
     cudaError_t e;
     TcGemm g = tc_gemm(kEpiHidden, m.gemmErr);
-    g.M = n; g.N = kHid; g.BN = 128; g.Mv = n; g.Nv = kHid;
+    g.M = n; g.N = kHid; g.BN = 128; g.Mv = n; g.Nv = kHid; g.ldh = kHid;
     g.K = kIn; g.KC = 64; g.kSlice = kIn;
-    g.bias = m.params + kB1; g.Z = f.z1; g.ldZ = kHid; g.Hb = f.h1; g.ldh = kHid; g.HT = f.h1T; g.ldht = f.ldT;
-    if ((e = gemm_tc(*f.aX, mp.bW1, g, s)) != cudaSuccess) return e;
-    g.K = kHid; g.KC = 64; g.kSlice = kHid;
-    g.bias = m.params + kB2; g.Z = f.z2; g.Hb = f.h2; g.HT = f.h2T;
-    if ((e = gemm_tc(*f.aH1, mp.bW2, g, s)) != cudaSuccess) return e;
-    g.bias = m.params + kB3; g.Z = f.z3; g.Hb = f.h3; g.HT = f.h3T;
-    if ((e = gemm_tc(*f.aH2, mp.bW3, g, s)) != cudaSuccess) return e;
+    g.bias = m.params + kB1; g.Hb = m.ph1;
+    if ((e = gemm_tc(mp.pX, mp.bW1, g, s)) != cudaSuccess) return e;
+    g.K = kHid; g.kSlice = kHid;
+    g.bias = m.params + kB2; g.Hb = m.ph2;
+    if ((e = gemm_tc(mp.pH1, mp.bW2, g, s)) != cudaSuccess) return e;
+    g.bias = m.params + kB3; g.Hb = m.ph3;
+    if ((e = gemm_tc(mp.pH2, mp.bW3, g, s)) != cudaSuccess) return e;
     g = tc_gemm(kEpiOut, m.gemmErr);
     g.M = n; g.N = 32; g.BN = 32; g.Mv = n; g.Nv = kOut;
     g.K = kHid; g.KC = 64; g.kSlice = kHid;
-    g.bias = m.params + kB4; g.C = f.out; g.ldc = kOut;
-    return gemm_tc(*f.aH3, mp.bW4, g, s);
+    g.bias = m.params + kB4; g.C = m.pout; g.ldc = kOut;
+    return gemm_tc(mp.pH3, mp.bW4, g, s);
 }
 
 // K slices of the weight-gradient products (K = the batch rows padded to 64):
@@ -545,72 +359,51 @@ int wgrad_slice(int K)
     return sl;
 }
 
-// Backward from dOut (m.dOut FP32, m.dOutB and m.dOutT BF16) to m.grads.  The
-// input gradients dZ3 -> dZ2 -> dZ1 form the chain; each layer's weight and bias
-// gradients need only that layer's dZ, so with a side stream they run beside the
-// chain (each in its own split-K and FP32 dZ buffers) and join it at the end.
-cudaError_t backward(Mlp& m, int n, cudaStream_t s, cudaStream_t side)
+// Forward, loss and input gradients of n rows (mlp_step.cuh), then the partials of
+// the weight gradients; *src is where the gradients are.
+cudaError_t step_products(Mlp& m, StepArgs a, cudaStream_t s, GradSource* src)
 {
     const TcMaps& mp = *m.maps;
-    float* G = m.grads;
-    cudaError_t e;
-    const int Kb = (n + 63) / 64 * 64;
-    const long long wsLayer = (long long)kMaxSplit * kHid * kHid;
-    const long long dzLayer = m.Ba * kHid;
-    cudaStream_t sw = side ? side : s;
-    // the side stream continues once the chain has produced the next dZ
-    auto fork = [&](int i) -> cudaError_t {
-        if (!side) return cudaSuccess;
-        cudaError_t r = cudaEventRecord(m.ev[i], s);
-        return r == cudaSuccess ? cudaStreamWaitEvent(side, m.ev[i], 0) : r;
-    };
-    TcGemm w = tc_gemm(kEpiWgrad, m.gemmErr);  // dW = dZ^T H_prev over the batch
-    w.K = Kb; w.KC = 64; w.kSlice = wgrad_slice(Kb);
-    TcGemm d = tc_gemm(kEpiDgrad, m.gemmErr);  // dZ_prev = (dZ W) * silu'(Z_prev)
-    d.M = n; d.N = kHid; d.BN = 128; d.Mv = n; d.Nv = kHid;
-    d.ldzp = kHid; d.ldc = kHid; d.ldh = kHid; d.ldht = m.Ba;
+    const int n = a.n;
+    const long long tiles = (n + kTcM - 1) / kTcM;
+    a.wp = m.wp;
+    a.params = m.params;
+    a.xT = m.xT; a.h1T = m.h1T; a.h2T = m.h2T; a.h3T = m.h3T;
+    a.dOutT = m.dOutT; a.dz3T = m.dz3T; a.dz2T = m.dz2T; a.dz1T = m.dz1T;
+    a.ld = m.Ba;
+    a.z = (float4*)m.z;
+    a.gradT = m.gradT;
+    a.loss = m.loss;
+    a.err = m.gemmErr;
+    mlp_step_kernel<<<(unsigned)tiles, kTcThreads, kTcSmem, s>>>(a);
+    note_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
 
-    // layer 4: dW4 = dOut^T H3, db4 = colsum(dOut) beside dZ3 = (dOut W4) * silu'(Z3)
-    if ((e = fork(0)) != cudaSuccess) return e;
-    TcGemm g = w;
-    g.M = kOut; g.N = kHid; g.BN = 128; g.Mv = kOut; g.Nv = kHid; g.C = G + kW4; g.ldc = kHid; g.ws = m.ws;
-    if ((e = gemm_tc(mp.aDOutT, mp.bH3T, g, sw)) != cudaSuccess) return e;
-    if ((e = colsum(m.dOut, n, kOut, kOut, G + kB4, sw)) != cudaSuccess) return e;
-    g = d;
-    g.K = kDOutPitch; g.KC = 32; g.kSlice = kDOutPitch; g.zp = m.z3; g.C = m.dzf; g.Hb = m.dz3; g.HT = m.dz3T;
-    if ((e = gemm_tc(mp.aDOut, mp.bW4T, g, s)) != cudaSuccess) return e;
-    // layers 3, 2: dW = dZ^T H_prev, db = colsum(dZ) beside dZ_prev
-    const CUtensorMap* aDzT[2] = {&mp.aDZ3T, &mp.aDZ2T};
-    const CUtensorMap* bHT[2] = {&mp.bH2T, &mp.bH1T};
-    const CUtensorMap* aDz[2] = {&mp.aDZ3, &mp.aDZ2};
-    const CUtensorMap* bWT[2] = {&mp.bW3T, &mp.bW2T};
-    const long long wOff[2] = {kW3, kW2}, bOff[2] = {kB3, kB2};
-    const float* zPrev[2] = {m.z2, m.z1};
-    bf16* dzPrev[2] = {m.dz2, nullptr};
-    bf16* dzPrevT[2] = {m.dz2T, m.dz1T};
-    for (int l = 0; l < 2; ++l) {
-        if ((e = fork(1 + l)) != cudaSuccess) return e;
-        g = w;
-        g.M = kHid; g.N = kHid; g.BN = 128; g.Mv = kHid; g.Nv = kHid; g.C = G + wOff[l]; g.ldc = kHid;
-        g.ws = m.ws + (1 + l) * wsLayer;
-        if ((e = gemm_tc(*aDzT[l], *bHT[l], g, sw)) != cudaSuccess) return e;
-        if ((e = colsum(m.dzf + l * dzLayer, n, kHid, kHid, G + bOff[l], sw)) != cudaSuccess) return e;
-        g = d;
-        g.K = kHid; g.KC = 64; g.kSlice = kHid; g.zp = zPrev[l]; g.C = m.dzf + (l + 1) * dzLayer;
-        g.Hb = dzPrev[l]; g.HT = dzPrevT[l];
-        if ((e = gemm_tc(*aDz[l], *bWT[l], g, s)) != cudaSuccess) return e;
+    const int Kb = (n + 63) / 64 * 64, slice = wgrad_slice(Kb), splits = (Kb + slice - 1) / slice;
+    const long long wsLayer = (long long)kMaxSplit * kHid * kHid;
+    WgradGroup W;
+    memset(&W, 0, sizeof(W));
+    const CUtensorMap* as[4] = {&mp.aDOutT, &mp.aDZ3T, &mp.aDZ2T, &mp.aDZ1T};
+    const CUtensorMap* bs[4] = {&mp.bH3T, &mp.bH2T, &mp.bH1T, &mp.bXT};
+    const int M[4] = {kOut, kHid, kHid, kHid}, N[4] = {kHid, kHid, kHid, kIn};
+    for (int l = 0; l < 4; ++l) {
+        W.a[l] = *as[l];
+        W.b[l] = *bs[l];
+        TcGemm& g = W.g[l];
+        g = tc_gemm(kEpiWgrad, m.gemmErr);
+        g.M = g.Mv = M[l]; g.N = g.Nv = N[l]; g.BN = 128;
+        g.K = Kb; g.KC = 64; g.kSlice = slice;
+        g.ws = m.ws + l * wsLayer;
+        W.nx[l] = (M[l] + kGtM - 1) / kGtM;
+        W.ny[l] = N[l] / 128;
+        W.first[l + 1] = W.first[l] + W.nx[l] * W.ny[l] * splits;
     }
-    // layer 1: dW1 = dZ1^T X, db1 (on the chain), then join the side stream
-    g = w;
-    g.M = kHid; g.N = kIn; g.BN = 128; g.Mv = kHid; g.Nv = kIn; g.C = G + kW1; g.ldc = kIn;
-    g.ws = m.ws + 3 * wsLayer;
-    if ((e = gemm_tc(mp.aDZ1T, mp.bXT, g, s)) != cudaSuccess) return e;
-    if ((e = colsum(m.dzf + 2 * dzLayer, n, kHid, kHid, G + kB1, s)) != cudaSuccess) return e;
-    if (side) {
-        if ((e = cudaEventRecord(m.ev[3], side)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, m.ev[3], 0)) != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    const size_t smem = (size_t)kGtStages * (kGtM + 128) * 64 * 2 + 64;
+    mlp_wgrad_kernel<<<W.first[4], kGtThreads, smem, s>>>(W);
+    note_launch();
+    *src = GradSource{m.ws, wsLayer, splits, m.gradT, m.Ba, n};
+    return cudaGetLastError();
 }
 
 // Reads and clears the products' error flag (call after a synchronisation).
@@ -643,31 +436,20 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
     m->Ba = Ba;
 #define A_(ptr, n) if (e == cudaSuccess) e = alloc_zero(&m->ptr, (n))
     A_(params, kNumParams); A_(grads, kNumParams); A_(m1, kNumParams); A_(m2, kNumParams);
-    A_(pb, kNumParams); A_(tw, kNumSlots * kSlot);
-    A_(xb, Ba * kXPitch); A_(xT, kXPitch * Ba); A_(xraw, Ba * kRaw); A_(yl, Ba); A_(yc, Ba);
-    A_(z1, Ba * kHid); A_(z2, Ba * kHid); A_(z3, Ba * kHid);
-    A_(h1, Ba * kHid); A_(h2, Ba * kHid); A_(h3, Ba * kHid);
+    A_(tw, kNumSlots * kSlot); A_(wp, (long long)kPkBytes);
+    A_(xT, kXPitch * Ba); A_(xraw, Ba * kRaw); A_(yl, Ba); A_(yc, Ba);
+    A_(z, 3 * Ba * kHid);
     A_(h1T, kHid * Ba); A_(h2T, kHid * Ba); A_(h3T, kHid * Ba);
-    A_(out, Ba * kOut); A_(dOut, Ba * kOut); A_(dOutB, Ba * kDOutPitch); A_(dOutT, kDOutTRows * Ba);
-    A_(dzf, 3 * Ba * kHid); A_(dz3, Ba * kHid); A_(dz2, Ba * kHid);
+    A_(out, Ba * kOut); A_(gradT, kGradRows * Ba); A_(dOutT, kDOutTRows * Ba);
     A_(dz3T, kHid * Ba); A_(dz2T, kHid * Ba); A_(dz1T, kHid * Ba);
-    A_(loss, 1); A_(step, 1); A_(gemmErr, 1);
+    A_(loss, 1); A_(step, 1); A_(finished, 1); A_(gemmErr, 1);
     A_(ws, 4ll * kMaxSplit * kHid * kHid);
 #undef A_
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking);
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&m->ev[i], cudaEventDisableTiming);
     if (e != cudaSuccess) return report_cuda_error(e, "surrogate network buffers");
     m->maps = new TcMaps();
     TcMaps& mp = *m->maps;
     const auto slot = [&](int k) { return m->tw + k * kSlot; };
 #define M_(map, p, R, C, ld, rows, kc) if (e == cudaSuccess) e = operand_map(&mp.map, p, R, C, ld, rows, kc)
-    M_(aX, m->xb, Ba, kXPitch, kXPitch, kGtM, 64);
-    M_(aH1, m->h1, Ba, kHid, kHid, kGtM, 64);
-    M_(aH2, m->h2, Ba, kHid, kHid, kGtM, 64);
-    M_(aH3, m->h3, Ba, kHid, kHid, kGtM, 64);
-    M_(aDOut, m->dOutB, Ba, kDOutPitch, kDOutPitch, kGtM, 32);
-    M_(aDZ3, m->dz3, Ba, kHid, kHid, kGtM, 64);
-    M_(aDZ2, m->dz2, Ba, kHid, kHid, kGtM, 64);
     M_(aDOutT, m->dOutT, kDOutTRows, Ba, Ba, kGtM, 64);
     M_(aDZ3T, m->dz3T, kHid, Ba, Ba, kGtM, 64);
     M_(aDZ2T, m->dz2T, kHid, Ba, Ba, kGtM, 64);
@@ -676,9 +458,6 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
     M_(bW2, slot(kSlotW2), kHid, kHid, kHid, 128, 64);
     M_(bW3, slot(kSlotW3), kHid, kHid, kHid, 128, 64);
     M_(bW4, slot(kSlotW4), kHid, kHid, kHid, 32, 64);
-    M_(bW4T, slot(kSlotW4T), kHid, kHid, kHid, 128, 32);
-    M_(bW3T, slot(kSlotW3T), kHid, kHid, kHid, 128, 64);
-    M_(bW2T, slot(kSlotW2T), kHid, kHid, kHid, 128, 64);
     M_(bH3T, m->h3T, kHid, Ba, Ba, 128, 64);
     M_(bH2T, m->h2T, kHid, Ba, Ba, 128, 64);
     M_(bH1T, m->h1T, kHid, Ba, Ba, 128, 64);
@@ -686,6 +465,10 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
 #undef M_
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtMaxSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtMaxSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     if (e != cudaSuccess) return report_cuda_error(e, "surrogate network tensor maps");
     return CBF_OK;
 }
@@ -694,14 +477,10 @@ void mlp_free(cbf_mlp* m)
 {
     if (m->exec) cudaGraphExecDestroy(m->exec);
     if (m->graph) cudaGraphDestroy(m->graph);
-    void* ptrs[] = {m->params, m->grads, m->m1, m->m2, m->pb, m->tw, m->xb, m->xT, m->xraw, m->yl, m->yc, m->z1,
-                    m->z2, m->z3, m->h1, m->h2, m->h3, m->h1T, m->h2T, m->h3T, m->out, m->dOut, m->dOutB,
-                    m->dOutT, m->dzf, m->dz3, m->dz2, m->dz3T, m->dz2T, m->dz1T, m->loss, m->ws, m->gemmErr,
-                    m->step, m->pxb, m->ph1, m->ph2, m->ph3, m->pout, m->wpack, m->tcErr};
+    void* ptrs[] = {m->params, m->grads, m->m1, m->m2, m->tw, m->wp, m->xT, m->xraw, m->yl, m->yc, m->z, m->h1T,
+                    m->h2T, m->h3T, m->out, m->gradT, m->dOutT, m->dz3T, m->dz2T, m->dz1T, m->loss, m->ws,
+                    m->gemmErr, m->step, m->finished, m->pxb, m->ph1, m->ph2, m->ph3, m->pout, m->tcErr};
     for (void* p : ptrs) cudaFree(p);
-    for (cudaEvent_t ev : m->ev)
-        if (ev) cudaEventDestroy(ev);
-    if (m->side) cudaStreamDestroy(m->side);
     delete m->maps;
     m->maps = nullptr;
 }
@@ -732,7 +511,7 @@ cbf_status upload_params(cbf_mlp* m, const float* host)
     cudaError_t e = cudaMemcpy(m->params, host, kNumParams * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = launch1d(kNumParams, 0, [&](unsigned b, int t) {
-            expand_params_kernel<<<b, t>>>(m->params, m->pb, m->tw, kNumParams);
+            expand_params_kernel<<<b, t>>>(m->params, m->tw, m->wp, kNumParams);
         });
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return report_cuda_error(e, "surrogate parameters");
@@ -822,23 +601,24 @@ cbf_status cbf_mlp_forward_backward(cbf_mlp* m, const float* hx, const float* hy
 {
     if (!m || !hx || !hyl || !hyc || n < 1 || n > m->B)
         return report_error(CBF_ERR_INVALID_ARG, "bad batch");
-    // encoded BF16 input rows and their transpose, zero for the rest of the last tile
-    const int rows = (n + kGtM - 1) / kGtM * kGtM;
     cudaError_t e = cudaMemcpy(m->xraw, hx, (size_t)n * kRaw * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = launch1d(rows, 0, [&](unsigned b, int t) {
-            encode_rows_kernel<<<b, t>>>(m->xraw, n, rows, m->encScale, m->xb, m->xT, m->Ba);
-        });
     if (e == cudaSuccess) e = cudaMemcpy(m->yl, hyl, (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(m->yc, hyc, (size_t)n * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(m->loss, 0, sizeof(float));
-    if (e == cudaSuccess) e = forward(*m, n, train_bufs(*m), 0);
-    if (e == cudaSuccess)
-        e = launch1d(rows, 0, [&](unsigned b, int t) {
-            loss_kernel<<<b, t>>>(m->out, m->yl, m->yc, n, rows, wLle, m->dOut, m->dOutB, m->dOutT, m->Ba,
-                                  m->loss);
-        });
-    if (e == cudaSuccess) e = backward(*m, n, 0, nullptr);
+    if (e == cudaSuccess) {
+        StepArgs a;
+        memset(&a, 0, sizeof(a));
+        a.X = m->xraw; a.yl = m->yl; a.yc = m->yc; a.N = n; a.n = n;
+        a.fs = m->encScale; a.wLle = wLle;
+        a.out = m->out;
+        GradSource src;
+        e = step_products(*m, a, 0, &src);
+        if (e == cudaSuccess) {
+            mlp_grads_kernel<<<kParamBlocks + kBiasBlocks, kParamThreads>>>(src, m->grads);
+            note_launch();
+            e = cudaGetLastError();
+        }
+    }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = gemm_status(*m);
     if (e == cudaSuccess && hloss) e = cudaMemcpy(hloss, m->loss, sizeof(float), cudaMemcpyDeviceToHost);
@@ -863,7 +643,7 @@ cbf_status cbf_mlp_train(cbf_mlp* m, const float* dX, const float* dYl, const in
     if (!s) return report_error(CBF_ERR_INVALID_ARG, "training needs a non-default stream");
     const int B = m->B;
     cudaError_t e = cudaSuccess;
-    if (!m->exec || m->gX != dX || m->gN != N || m->gLr != lr || m->gHorizon != horizon ||
+    if (!m->exec || m->gX != dX || m->gYl != dYl || m->gYc != (const int*)dYc || m->gN != N || m->gLr != lr || m->gHorizon != horizon ||
         m->gW != wLle || m->gSeed != m->seed || m->gScale != m->encScale) {
         if (m->exec) cudaGraphExecDestroy(m->exec);
         if (m->graph) cudaGraphDestroy(m->graph);
@@ -871,25 +651,17 @@ cbf_status cbf_mlp_train(cbf_mlp* m, const float* dX, const float* dYl, const in
         m->graph = nullptr;
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return report_cuda_error(e, "begin capture of the training step");
-        cudaError_t ce = launch1d(B, s, [&](unsigned b, int t) {
-            gather_kernel<<<b, t, 0, s>>>(dX, dYl, (const int*)dYc, N, B, m->step, m->seed, m->encScale,
-                                          m->xb, m->xT, m->Ba, m->yl, m->yc);
-        });
-        const int rows = (B + kGtM - 1) / kGtM * kGtM;
-        if (ce == cudaSuccess) ce = forward(*m, B, train_bufs(*m), s);
-        if (ce == cudaSuccess)
-            ce = launch1d(rows, s, [&](unsigned b, int t) {
-                loss_kernel<<<b, t, 0, s>>>(m->out, m->yl, m->yc, B, rows, wLle, m->dOut, m->dOutB, m->dOutT,
-                                            m->Ba, m->loss);
-            });
-        if (ce == cudaSuccess) ce = backward(*m, B, s, m->side);
-        if (ce == cudaSuccess)
-            ce = launch1d(kNumParams, s, [&](unsigned b, int t) {
-                adam_kernel<<<b, t, 0, s>>>(m->params, m->grads, m->m1, m->m2, m->pb, m->tw, kNumParams, lr,
-                                            horizon, 0.9f, 0.999f, 1e-8f, m->step);
-            });
+        StepArgs a;
+        memset(&a, 0, sizeof(a));
+        a.X = dX; a.yl = dYl; a.yc = (const int*)dYc; a.N = N; a.n = B;
+        a.draw = 1; a.step = m->step; a.seed = m->seed;
+        a.fs = m->encScale; a.wLle = wLle;
+        GradSource src;
+        cudaError_t ce = step_products(*m, a, s, &src);
         if (ce == cudaSuccess) {
-            bump_kernel<<<1, 1, 0, s>>>(m->step);
+            mlp_adam_kernel<<<kParamBlocks + kBiasBlocks, kParamThreads, 0, s>>>(src, m->params, m->m1, m->m2, m->tw,
+                                                                                 m->wp, lr, horizon, 0.9f, 0.999f,
+                                                                                 1e-8f, m->step, m->finished);
             note_launch();
             ce = cudaGetLastError();
         }
@@ -904,6 +676,8 @@ cbf_status cbf_mlp_train(cbf_mlp* m, const float* dX, const float* dYl, const in
         e = cudaGraphInstantiate(&m->exec, gph, 0);
         if (e != cudaSuccess) return report_cuda_error(e, "instantiate the training graph");
         m->gX = dX;
+        m->gYl = dYl;
+        m->gYc = (const int*)dYc;
         m->gN = N;
         m->gLr = lr;
         m->gHorizon = horizon;
@@ -938,9 +712,9 @@ cbf_status cbf_mlp_predict(cbf_mlp* m, const float* dX, int64_t N, float lleMean
     for (long long r0 = 0; r0 < N && e == cudaSuccess; r0 += kPredRows) {
         const int n = (int)((N - r0) < kPredRows ? (N - r0) : kPredRows);
         e = launch1d(n, s, [&](unsigned b, int t) {
-            encode_rows_kernel<<<b, t, 0, s>>>(dX + r0 * kRaw, n, n, m->encScale, m->pxb, nullptr, 0);
+            encode_rows_kernel<<<b, t, 0, s>>>(dX + r0 * kRaw, n, m->encScale, m->pxb);
         });
-        if (e == cudaSuccess) e = forward(*m, n, pred_bufs(*m), s);
+        if (e == cudaSuccess) e = forward(*m, n, s);
         if (e == cudaSuccess)
             e = launch1d(n, s, [&](unsigned b, int t) {
                 head_kernel<<<b, t, 0, s>>>(m->pout, n, lleMean, lleStd, dLle ? dLle + r0 : nullptr,
@@ -1004,19 +778,15 @@ cudaError_t mlp_features(const FeatureSpec& f, const long long* idx, long long n
     return launch1d(n, s, [&](unsigned b, int t) { features_kernel<<<b, t, 0, s>>>(f, idx, n, X); });
 }
 
-// One fused tcgen05 kernel over the whole grid (mlp_tc.cuh), after packing the
-// current BF16 weights into the operand layout.  A wait that ran out inside
-// the kernel is reported as cudaErrorLaunchTimeout.
+// One fused tcgen05 kernel over the whole grid (mlp_tc.cuh).  A wait that ran out
+// inside the kernel is reported as cudaErrorLaunchTimeout.
 cudaError_t mlp_predict_grid(cbf_mlp* m, const FeatureSpec& f, long long nPoints, float lleMean,
                              float lleStd, double* lle, int* cls, float* conf, cudaStream_t s)
 {
     if (nPoints <= 0) return cudaSuccess;
     cudaError_t e = cudaSuccess;
-    if (!m->wpack) e = cudaMalloc((void**)&m->wpack, kTcPackBytes);
-    if (e == cudaSuccess && !m->tcErr) e = cudaMalloc((void**)&m->tcErr, sizeof(int));
+    if (!m->tcErr) e = cudaMalloc((void**)&m->tcErr, sizeof(int));
     if (e != cudaSuccess) return e;
-    e = launch1d(kTcPackBytes / 2, s,
-                 [&](unsigned b, int t) { tc_pack_kernel<<<b, t, 0, s>>>(m->pb, (bf16*)m->wpack); });
     if (e == cudaSuccess) e = cudaMemsetAsync(m->tcErr, 0, sizeof(int), s);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_predict_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
@@ -1026,7 +796,7 @@ cudaError_t mlp_predict_grid(cbf_mlp* m, const FeatureSpec& f, long long nPoints
     if (e != cudaSuccess) return e;
     const long long tiles = (nPoints + kTcM - 1) / kTcM;
     const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-    mlp_predict_tc_kernel<<<grid, kTcThreads, kTcSmem, s>>>(f, nPoints, m->encScale, m->wpack, m->params, lleMean,
+    mlp_predict_tc_kernel<<<grid, kTcThreads, kTcSmem, s>>>(f, nPoints, m->encScale, m->wp, m->params, lleMean,
                                                             lleStd, lle, cls, conf, m->tcErr);
     note_launch();
     e = cudaGetLastError();

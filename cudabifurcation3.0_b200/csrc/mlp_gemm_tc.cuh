@@ -1,15 +1,14 @@
-// Matrix products of the surrogate network's training step (and of the
-// prediction of explicit feature rows) on the 5th-generation tensor cores.
+// Matrix products of the surrogate network's weight gradients and of the prediction
+// of explicit feature rows on the 5th-generation tensor cores.
 // Included by mlp.cu after mlp_tc.cuh, inside its anonymous namespace (uses its
 // descriptor, mbarrier and tensor-memory helpers, silu and silu_grad).
 //
 // One kernel form computes every product: a 128 x BN tile of
 //     D = A[M x K] * B[N x K]^T
-// with both operands K-contiguous BF16 matrices in global memory.  The
-// transposed operands that backpropagation needs are written as extra outputs
-// by the kernels that produce them -- H^T and dZ^T by this kernel's epilogues,
-// X^T by the minibatch gather, dOut^T by the loss, W^T by the Adam step -- so no
-// product ever reads a matrix across its rows.
+// with both operands K-contiguous BF16 matrices in global memory.  The transposed
+// operands of the weight gradients (X^T, H^T, dOut^T, dZ^T) are written by the
+// kernel that produces them (mlp_step.cuh), so no product ever reads a matrix
+// across its rows.
 //
 // Operands reach shared memory by TMA (cp.async.bulk.tensor, 4-D tensor maps)
 // directly in the UMMA K-major no-swizzle core-matrix layout.  The tensor map of
@@ -30,13 +29,11 @@
 // mbarrier; longer K slices run in passes of four chunks.  The eight warps then
 // read the accumulator (tcgen05.ld.32x32b.x32, warp w: lanes 32(w%4).., every
 // other 32-column chunk) and apply the epilogue:
-//   kEpiHidden  z = acc + bias -> Z (FP32), h = SiLU(z) -> H (BF16) and H^T
+//   kEpiHidden  h = SiLU(acc + bias) -> H (BF16)
 //   kEpiOut     acc + bias -> C (FP32), the columns n < Nv
-//   kEpiDgrad   d = acc * SiLU'(zp) -> C (FP32), H (BF16), H^T (BF16)
-//   kEpiWgrad   acc -> C, or the K slice's partial into ws (split K; the
-//               slices are added in order by splitk_reduce_kernel)
-// Rows m >= Mv of a tile write zeros into H^T, so that a later product whose K
-// runs over the padded batch adds nothing for them.  Every mbarrier wait is
+//   kEpiWgrad   the K slice's partial into ws (split K; the slices are added in
+//               order by the kernel that uses the gradients)
+// Every mbarrier wait is
 // bounded: a wait that runs out drains the copies and products in flight (again
 // bounded), sets the error flag and frees the tensor memory.  (mlp.cu includes
 // <cuda.h> for the tensor-map types.)
@@ -46,7 +43,7 @@ constexpr int kGtThreads = 256;
 constexpr int kGtStages = 4;
 constexpr size_t kGtMaxSmem = (size_t)kGtStages * (kGtM + 256) * 64 * 2 + 128;
 
-enum { kEpiHidden = 0, kEpiOut = 1, kEpiDgrad = 2, kEpiWgrad = 3 };
+enum { kEpiHidden = 0, kEpiOut = 1, kEpiWgrad = 2 };
 
 struct TcGemm {
     int M, N, K;     // rows computed (tiles of 128), columns (a multiple of BN), reduction length
@@ -55,17 +52,11 @@ struct TcGemm {
     int Mv, Nv;      // rows and columns of the result that exist
     int mode;
     const float* bias;
-    const float* zp;  // kEpiDgrad: pre-activation whose SiLU derivative scales the product
-    long long ldzp;
-    float* Z;         // kEpiHidden: pre-activation (after bias), row-major
-    long long ldZ;
     float* C;         // FP32 result, row-major
     long long ldc;
     bf16* Hb;         // BF16 result, row-major
     long long ldh;
-    bf16* HT;         // BF16 result transposed: HT[n * ldht + m]
-    long long ldht;
-    float* ws;        // kEpiWgrad with splits: ws[(z * Mv + m) * Nv + n]
+    float* ws;        // kEpiWgrad: ws[(z * Mv + m) * Nv + n]
     int* err;
 };
 
@@ -96,13 +87,14 @@ __device__ __forceinline__ void store_bf16x32(bf16* p, const float (&v)[32])
                        pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
 }
 
-__global__ void __launch_bounds__(kGtThreads, 1)
-    gemm_tc_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const TcGemm g)
+// Tile (bx, by) of the product, K slice bz; `partial`: into the slice's part of ws.
+__device__ __forceinline__ void gemm_tile(const CUtensorMap* ta, const CUtensorMap* tb, const TcGemm& g, int bx, int by,
+                                          int bz, bool partial)
 {
     extern __shared__ __align__(1024) unsigned char gsm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kGtM, n0 = blockIdx.y * g.BN;
-    const int kBeg = blockIdx.z * g.kSlice;
+    const int m0 = bx * kGtM, n0 = by * g.BN;
+    const int kBeg = bz * g.kSlice;
     const int kEnd = min(g.K, kBeg + g.kSlice);
     const int nch = (kEnd - kBeg) / g.KC;
     const int S = nch < kGtStages ? nch : kGtStages;
@@ -141,8 +133,8 @@ __global__ void __launch_bounds__(kGtThreads, 1)
                 const uint32_t fb = smem_u32(&bars[j]);
                 const int kg = (kBeg + (c0 + j) * g.KC) >> 3;
                 mbar_expect_tx(fb, stBytes);
-                tma_load4(base + (uint32_t)j * stBytes, &ta, 0, 0, m0 >> 3, kg, fb);
-                tma_load4(base + (uint32_t)j * stBytes + aBytes, &tb, 0, 0, n0 >> 3, kg, fb);
+                tma_load4(base + (uint32_t)j * stBytes, ta, 0, 0, m0 >> 3, kg, fb);
+                tma_load4(base + (uint32_t)j * stBytes + aBytes, tb, 0, 0, n0 >> 3, kg, fb);
             }
             int j = 0;
             for (; j < cn; ++j) {
@@ -184,44 +176,16 @@ __global__ void __launch_bounds__(kGtThreads, 1)
             const int nb = n0 + ch * 32;
             if (g.mode == kEpiHidden) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] += g.bias[nb + j];
-                if (rv && g.Z) store_f32x32(g.Z + row * g.ldZ + nb, v);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
-                if (rv && g.Hb) store_bf16x32(g.Hb + row * g.ldh + nb, v);
-                if (g.HT) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        g.HT[(long long)(nb + j) * g.ldht + row] = __float2bfloat16_rn(rv ? v[j] : 0.0f);
-                }
-            } else if (g.mode == kEpiDgrad) {
-                if (rv) {
-                    const float4* z4 = reinterpret_cast<const float4*>(g.zp + row * g.ldzp + nb);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float4 z = z4[i];
-                        v[4 * i] *= silu_grad(z.x);
-                        v[4 * i + 1] *= silu_grad(z.y);
-                        v[4 * i + 2] *= silu_grad(z.z);
-                        v[4 * i + 3] *= silu_grad(z.w);
-                    }
-                    if (g.C) store_f32x32(g.C + row * g.ldc + nb, v);
-                    if (g.Hb) store_bf16x32(g.Hb + row * g.ldh + nb, v);
-                }
-                if (g.HT) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        g.HT[(long long)(nb + j) * g.ldht + row] = __float2bfloat16_rn(rv ? v[j] : 0.0f);
-                }
+                for (int j = 0; j < 32; ++j) v[j] = silu(v[j] + g.bias[nb + j]);
+                if (rv) store_bf16x32(g.Hb + row * g.ldh + nb, v);
             } else if (g.mode == kEpiOut) {
                 if (rv)
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (nb + j < g.Nv) g.C[row * g.ldc + nb + j] = v[j] + g.bias[nb + j];
             } else if (rv) {  // kEpiWgrad
-                float* dst = gridDim.z > 1 ? g.ws + ((long long)blockIdx.z * g.Mv + row) * g.Nv
-                                           : g.C + row * g.ldc;
-                const long long ld = gridDim.z > 1 ? g.Nv : g.ldc;
+                float* dst = partial ? g.ws + ((long long)bz * g.Mv + row) * g.Nv : g.C + row * g.ldc;
+                const long long ld = partial ? g.Nv : g.ldc;
                 if (nb + 32 <= g.Nv && (ld & 3) == 0 && ((uintptr_t)dst & 15) == 0) {
                     store_f32x32(dst + nb, v);
                 } else {
@@ -238,6 +202,12 @@ __global__ void __launch_bounds__(kGtThreads, 1)
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     if (bad && tid == 0) atomicExch(g.err, 1);
+}
+
+__global__ void __launch_bounds__(kGtThreads, 1)
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const TcGemm g)
+{
+    gemm_tile(&ta, &tb, g, blockIdx.x, blockIdx.y, blockIdx.z, false);
 }
 
 // ---- host side -------------------------------------------------------------
@@ -286,24 +256,16 @@ cudaError_t operand_map(CUtensorMap* map, const bf16* p, long long R, long long 
 }
 
 // One product: A through `ta` (128-row tiles, KC-wide), B through `tb` (BN-row
-// tiles, KC-wide); split-K partials are added in slice order afterwards.
+// tiles, KC-wide).
 cudaError_t gemm_tc(const CUtensorMap& ta, const CUtensorMap& tb, const TcGemm& g, cudaStream_t s)
 {
     if (g.M <= 0 || g.Mv <= 0) return cudaSuccess;
     if (g.BN < 16 || g.BN > 256 || g.BN % 16 || g.N % g.BN || (g.KC != 16 && g.KC != 32 && g.KC != 64) ||
-        g.K <= 0 || g.K % g.KC || g.kSlice <= 0 || g.kSlice % g.KC || g.Nv > g.N ||
-        ((g.mode == kEpiHidden || g.mode == kEpiDgrad) && g.BN % 32))
+        g.K <= 0 || g.K % g.KC || g.kSlice != g.K || g.Nv > g.N || (g.mode == kEpiHidden && g.BN % 32))
         return cudaErrorInvalidValue;
-    const int splits = (g.K + g.kSlice - 1) / g.kSlice;
-    if (splits > 1 && (g.mode != kEpiWgrad || !g.ws)) return cudaErrorInvalidValue;
-    const dim3 grid((unsigned)((g.M + kGtM - 1) / kGtM), (unsigned)(g.N / g.BN), (unsigned)splits);
+    const dim3 grid((unsigned)((g.M + kGtM - 1) / kGtM), (unsigned)(g.N / g.BN), 1);
     const size_t smem = (size_t)kGtStages * (kGtM + g.BN) * g.KC * 2 + 64;
     gemm_tc_kernel<<<grid, kGtThreads, smem, s>>>(ta, tb, g);
-    note_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || splits == 1) return e;
-    const long long MN = (long long)g.Mv * g.Nv;
-    splitk_reduce_kernel<<<(unsigned)((MN + 255) / 256), 256, 0, s>>>(g.ws, splits, g.Mv, g.Nv, g.C, g.ldc, 1);
     note_launch();
     return cudaGetLastError();
 }

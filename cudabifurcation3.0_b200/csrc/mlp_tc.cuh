@@ -20,8 +20,8 @@
 //   (k / 8) * (R * 16) + (r / 8) * 128 + (r % 8) * 16 + (k % 8) * 2  bytes,
 // i.e. leading-dimension byte offset (between the two 8-k halves of one
 // K = 16 MMA) R * 16, stride-dimension byte offset (between 8-row groups) 128.
-// The weights are packed once per call into exactly this layout in global
-// memory, so each layer's copy is a plain contiguous bulk copy.
+// The weights are kept in exactly this layout in global memory (refreshed with the
+// parameters), so each layer's copy is a plain contiguous bulk copy.
 
 constexpr int kTcM = 128;        // grid points per tile (MMA M, tensor-memory lanes)
 constexpr int kTcThreads = 512;  // 16 warps: four per tensor-memory lane quarter
@@ -31,7 +31,6 @@ constexpr uint32_t kTcABytes = kTcM * kHid * 2;      // 65536
 constexpr uint32_t kTcBBytes = kHid * kHid * 2;      // 131072
 constexpr uint32_t kTcW1Bytes = kHid * kIn * 2;      // 65536
 constexpr uint32_t kTcW4Bytes = kTcN4 * kHid * 2;    // 16384
-constexpr uint32_t kTcPackBytes = kTcW1Bytes + 2 * kTcBBytes + kTcW4Bytes;
 constexpr size_t kTcSmem = kTcABytes + kTcBBytes + 64;
 constexpr long long kTcSpin = 1ll << 22;  // polls of an mbarrier before giving up (~0.3 s)
 
@@ -143,34 +142,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-
-// The BF16 weights (flat layout of the parameter buffer) in the shared-memory
-// operand layout: W1 (256 x 4, K padded to 16), W2, W3 (256 x 256), W4 (17 x
-// 256, rows padded to 32), one 2-byte element per thread.
-__global__ void tc_pack_kernel(const bf16* __restrict__ pb, bf16* __restrict__ out)
-{
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= kTcPackBytes / 2) return;
-    uint32_t o = (uint32_t)e * 2;
-    int R, K;
-    long long src;
-    if (o < kTcW1Bytes) {
-        R = kHid; K = kIn; src = kW1;
-    } else if ((o -= kTcW1Bytes) < kTcBBytes) {
-        R = kHid; K = kHid; src = kW2;
-    } else if ((o -= kTcBBytes) < kTcBBytes) {
-        R = kHid; K = kHid; src = kW3;
-    } else {
-        o -= kTcBBytes;
-        R = kTcN4; K = kHid; src = kW4;
-    }
-    const int kc = (int)(o / (uint32_t)(R * 16));
-    const uint32_t rem = o % (uint32_t)(R * 16);
-    const int r = (int)(rem / 128) * 8 + (int)((rem % 128) / 16);
-    const int k = kc * 8 + (int)((rem % 16) / 2);
-    const int rows = (src == kW4) ? kOut : kHid;
-    out[e] = (r < rows && k < K) ? pb[src + (long long)r * K + k] : __float2bfloat16_rn(0.0f);
-}
 
 // Issue the MMAs of one layer (one thread) once its weights have arrived.
 __device__ __forceinline__ void tc_issue(uint32_t tmem, uint32_t aAddr, uint32_t bAddr, int slices, uint32_t lboB,
