@@ -51,7 +51,6 @@ constexpr long long kSlot = (long long)kHid * kHid;
 enum { kSlotW1 = 0, kSlotW2, kSlotW3, kSlotW4, kNumSlots };
 constexpr int kXPitch = kIn;   // BF16 first-layer input rows
 constexpr int kDOutPitch = 32;  // output gradients as an operand: 17 values padded to K = 32
-constexpr int kDOutTRows = 128; // rows of dOut^T (17 used): one full 128-row operand tile
 
 // SiLU z * sigmoid(z) and its derivative.  The sigmoid's quotient uses the
 // approximate reciprocal (__fdividef: a few ulp of FP32, far below the BF16
@@ -246,11 +245,9 @@ cudaError_t launch1d(long long n, cudaStream_t s, F f)
 
 // ---------------------------------------------------------------------------
 
-// Tensor maps of every operand the products read (fixed buffers, built once).
+// Tensor maps of the products of explicit feature rows (fixed buffers, built once).
 struct TcMaps {
-    // weight gradients: A operands dOut^T, dZ^T (128-row tiles), B operands H^T, X^T
-    CUtensorMap aDOutT, aDZ3T, aDZ2T, aDZ1T, bH3T, bH2T, bH1T, bXT;
-    // explicit feature rows: A operands (the prediction workspace), B operands W
+    // A operands (128-row tiles of the prediction workspace), B operands W
     CUtensorMap pX, pH1, pH2, pH3, bW1, bW2, bW3, bW4;
 };
 
@@ -265,16 +262,14 @@ struct Mlp {
     float* m2 = nullptr;
     bf16* tw = nullptr;       // row-major BF16 weights (products of explicit rows)
     unsigned char* wp = nullptr;  // BF16 weights in the shared-memory operand layout (kPkBytes)
-    // batch buffers ("T": transposed, pitch Ba)
+    // batch buffers
     float* xraw = nullptr;     // raw feature rows and labels of cbf_mlp_forward_backward
     float* yl = nullptr;
     int* yc = nullptr;
-    bf16* xT = nullptr;
+    unsigned char* ops = nullptr;  // the step kernel's operands, tile by tile
     float* z = nullptr;        // pre-activations, in the step kernel's own order
-    bf16 *h1T = nullptr, *h2T = nullptr, *h3T = nullptr;
     float* out = nullptr;
-    float* gradT = nullptr;    // FP32 dOut, dZ3, dZ2, dZ1 for the bias gradients
-    bf16 *dOutT = nullptr, *dz3T = nullptr, *dz2T = nullptr, *dz1T = nullptr;
+    float* gradT = nullptr;    // FP32 dOut, dZ3, dZ2, dZ1, transposed, for the bias gradients
     float* loss = nullptr;
     float* ws = nullptr;      // split-K partials, one region per weight gradient
     int* gemmErr = nullptr;   // set by a kernel whose bounded wait ran out
@@ -334,24 +329,23 @@ cudaError_t forward(Mlp& m, int n, cudaStream_t s)
     cudaError_t e;
     TcGemm g = tc_gemm(kEpiHidden, m.gemmErr);
     g.M = n; g.N = kHid; g.BN = 128; g.Mv = n; g.Nv = kHid; g.ldh = kHid;
-    g.K = kIn; g.KC = 64; g.kSlice = kIn;
+    g.K = kIn; g.KC = 64;
     g.bias = m.params + kB1; g.Hb = m.ph1;
     if ((e = gemm_tc(mp.pX, mp.bW1, g, s)) != cudaSuccess) return e;
-    g.K = kHid; g.kSlice = kHid;
+    g.K = kHid;
     g.bias = m.params + kB2; g.Hb = m.ph2;
     if ((e = gemm_tc(mp.pH1, mp.bW2, g, s)) != cudaSuccess) return e;
     g.bias = m.params + kB3; g.Hb = m.ph3;
     if ((e = gemm_tc(mp.pH2, mp.bW3, g, s)) != cudaSuccess) return e;
     g = tc_gemm(kEpiOut, m.gemmErr);
     g.M = n; g.N = 32; g.BN = 32; g.Mv = n; g.Nv = kOut;
-    g.K = kHid; g.KC = 64; g.kSlice = kHid;
+    g.K = kHid; g.KC = 64;
     g.bias = m.params + kB4; g.C = m.pout; g.ldc = kOut;
     return gemm_tc(mp.pH3, mp.bW4, g, s);
 }
 
 // K slices of the weight-gradient products (K = the batch rows padded to 64):
 // 256 rows each, wider when that would exceed kMaxSplit slices.
-constexpr int kMaxSplit = 16;
 int wgrad_slice(int K)
 {
     int sl = 256;
@@ -363,13 +357,11 @@ int wgrad_slice(int K)
 // the weight gradients; *src is where the gradients are.
 cudaError_t step_products(Mlp& m, StepArgs a, cudaStream_t s, GradSource* src)
 {
-    const TcMaps& mp = *m.maps;
     const int n = a.n;
     const long long tiles = (n + kTcM - 1) / kTcM;
     a.wp = m.wp;
     a.params = m.params;
-    a.xT = m.xT; a.h1T = m.h1T; a.h2T = m.h2T; a.h3T = m.h3T;
-    a.dOutT = m.dOutT; a.dz3T = m.dz3T; a.dz2T = m.dz2T; a.dz1T = m.dz1T;
+    a.ops = m.ops;
     a.ld = m.Ba;
     a.z = (float4*)m.z;
     a.gradT = m.gradT;
@@ -382,25 +374,28 @@ cudaError_t step_products(Mlp& m, StepArgs a, cudaStream_t s, GradSource* src)
 
     const int Kb = (n + 63) / 64 * 64, slice = wgrad_slice(Kb), splits = (Kb + slice - 1) / slice;
     const long long wsLayer = (long long)kMaxSplit * kHid * kHid;
-    WgradGroup W;
+    WgradArgs W;
     memset(&W, 0, sizeof(W));
-    const CUtensorMap* as[4] = {&mp.aDOutT, &mp.aDZ3T, &mp.aDZ2T, &mp.aDZ1T};
-    const CUtensorMap* bs[4] = {&mp.bH3T, &mp.bH2T, &mp.bH1T, &mp.bXT};
+    const uint32_t as[4] = {kOpDOut, kOpDZ3, kOpDZ2, kOpDZ1}, bs[4] = {kOpH3, kOpH2, kOpH1, kOpX};
     const int M[4] = {kOut, kHid, kHid, kHid}, N[4] = {kHid, kHid, kHid, kIn};
+    int ctas = 0;
     for (int l = 0; l < 4; ++l) {
-        W.a[l] = *as[l];
-        W.b[l] = *bs[l];
-        TcGemm& g = W.g[l];
-        g = tc_gemm(kEpiWgrad, m.gemmErr);
-        g.M = g.Mv = M[l]; g.N = g.Nv = N[l]; g.BN = 128;
-        g.K = Kb; g.KC = 64; g.kSlice = slice;
-        g.ws = m.ws + l * wsLayer;
-        W.nx[l] = (M[l] + kGtM - 1) / kGtM;
-        W.ny[l] = N[l] / 128;
-        W.first[l + 1] = W.first[l] + W.nx[l] * W.ny[l] * splits;
+        WgradProduct& p = W.p[l];
+        p.a = as[l];
+        p.b = bs[l];
+        p.aBytes = l == 0 ? kTcM * kDOutPitch * 2 : kWgHalf;
+        p.M = M[l];
+        p.N = N[l];
+        p.nx = (M[l] + kTcM - 1) / kTcM;
+        p.first = ctas;
+        p.ws = m.ws + l * wsLayer;
+        ctas += p.nx * splits;
     }
-    const size_t smem = (size_t)kGtStages * (kGtM + 128) * 64 * 2 + 64;
-    mlp_wgrad_kernel<<<W.first[4], kGtThreads, smem, s>>>(W);
+    W.ops = m.ops;
+    W.K = Kb;
+    W.slice = slice;
+    W.err = m.gemmErr;
+    mlp_wgrad_kernel<<<ctas, kWgThreads, kWgSmem, s>>>(W);
     note_launch();
     *src = GradSource{m.ws, wsLayer, splits, m.gradT, m.Ba, n};
     return cudaGetLastError();
@@ -437,11 +432,9 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
 #define A_(ptr, n) if (e == cudaSuccess) e = alloc_zero(&m->ptr, (n))
     A_(params, kNumParams); A_(grads, kNumParams); A_(m1, kNumParams); A_(m2, kNumParams);
     A_(tw, kNumSlots * kSlot); A_(wp, (long long)kPkBytes);
-    A_(xT, kXPitch * Ba); A_(xraw, Ba * kRaw); A_(yl, Ba); A_(yc, Ba);
-    A_(z, 3 * Ba * kHid);
-    A_(h1T, kHid * Ba); A_(h2T, kHid * Ba); A_(h3T, kHid * Ba);
-    A_(out, Ba * kOut); A_(gradT, kGradRows * Ba); A_(dOutT, kDOutTRows * Ba);
-    A_(dz3T, kHid * Ba); A_(dz2T, kHid * Ba); A_(dz1T, kHid * Ba);
+    A_(xraw, Ba * kRaw); A_(yl, Ba); A_(yc, Ba);
+    A_(ops, Ba / kTcM * kOpTile); A_(z, 3 * Ba * kHid);
+    A_(out, Ba * kOut); A_(gradT, kGradRows * Ba);
     A_(loss, 1); A_(step, 1); A_(finished, 1); A_(gemmErr, 1);
     A_(ws, 4ll * kMaxSplit * kHid * kHid);
 #undef A_
@@ -450,23 +443,15 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
     TcMaps& mp = *m->maps;
     const auto slot = [&](int k) { return m->tw + k * kSlot; };
 #define M_(map, p, R, C, ld, rows, kc) if (e == cudaSuccess) e = operand_map(&mp.map, p, R, C, ld, rows, kc)
-    M_(aDOutT, m->dOutT, kDOutTRows, Ba, Ba, kGtM, 64);
-    M_(aDZ3T, m->dz3T, kHid, Ba, Ba, kGtM, 64);
-    M_(aDZ2T, m->dz2T, kHid, Ba, Ba, kGtM, 64);
-    M_(aDZ1T, m->dz1T, kHid, Ba, Ba, kGtM, 64);
     M_(bW1, slot(kSlotW1), kHid, kHid, kHid, 128, 64);
     M_(bW2, slot(kSlotW2), kHid, kHid, kHid, 128, 64);
     M_(bW3, slot(kSlotW3), kHid, kHid, kHid, 128, 64);
     M_(bW4, slot(kSlotW4), kHid, kHid, kHid, 32, 64);
-    M_(bH3T, m->h3T, kHid, Ba, Ba, 128, 64);
-    M_(bH2T, m->h2T, kHid, Ba, Ba, 128, 64);
-    M_(bH1T, m->h1T, kHid, Ba, Ba, 128, 64);
-    M_(bXT, m->xT, kXPitch, Ba, Ba, 128, 64);
 #undef M_
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtMaxSmem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGtMaxSmem);
+        e = cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
     if (e != cudaSuccess) return report_cuda_error(e, "surrogate network tensor maps");
@@ -477,8 +462,8 @@ void mlp_free(cbf_mlp* m)
 {
     if (m->exec) cudaGraphExecDestroy(m->exec);
     if (m->graph) cudaGraphDestroy(m->graph);
-    void* ptrs[] = {m->params, m->grads, m->m1, m->m2, m->tw, m->wp, m->xT, m->xraw, m->yl, m->yc, m->z, m->h1T,
-                    m->h2T, m->h3T, m->out, m->gradT, m->dOutT, m->dz3T, m->dz2T, m->dz1T, m->loss, m->ws,
+    void* ptrs[] = {m->params, m->grads, m->m1, m->m2, m->tw, m->wp, m->ops, m->xraw, m->yl, m->yc, m->z,
+                    m->out, m->gradT, m->loss, m->ws,
                     m->gemmErr, m->step, m->finished, m->pxb, m->ph1, m->ph2, m->ph3, m->pout, m->tcErr};
     for (void* p : ptrs) cudaFree(p);
     delete m->maps;

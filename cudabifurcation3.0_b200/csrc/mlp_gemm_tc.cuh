@@ -1,14 +1,11 @@
-// Matrix products of the surrogate network's weight gradients and of the prediction
-// of explicit feature rows on the 5th-generation tensor cores.
+// Matrix products of the prediction of explicit feature rows on the 5th-generation
+// tensor cores (the training step has kernels of its own, mlp_step.cuh).
 // Included by mlp.cu after mlp_tc.cuh, inside its anonymous namespace (uses its
-// descriptor, mbarrier and tensor-memory helpers, silu and silu_grad).
+// descriptor, mbarrier and tensor-memory helpers, silu).
 //
 // One kernel form computes every product: a 128 x BN tile of
 //     D = A[M x K] * B[N x K]^T
-// with both operands K-contiguous BF16 matrices in global memory.  The transposed
-// operands of the weight gradients (X^T, H^T, dOut^T, dZ^T) are written by the
-// kernel that produces them (mlp_step.cuh), so no product ever reads a matrix
-// across its rows.
+// with both operands K-contiguous BF16 matrices in global memory.
 //
 // Operands reach shared memory by TMA (cp.async.bulk.tensor, 4-D tensor maps)
 // directly in the UMMA K-major no-swizzle core-matrix layout.  The tensor map of
@@ -26,13 +23,11 @@
 // mbarrier each), then for each chunk, once it has landed, the KC/16
 // tcgen05.mma.cta_group::1.kind::f16 instructions (M 128, N BN) into an FP32
 // accumulator of BN tensor-memory columns, and commits them to a "done"
-// mbarrier; longer K slices run in passes of four chunks.  The eight warps then
+// mbarrier; a longer K runs in passes of four chunks.  The eight warps then
 // read the accumulator (tcgen05.ld.32x32b.x32, warp w: lanes 32(w%4).., every
 // other 32-column chunk) and apply the epilogue:
 //   kEpiHidden  h = SiLU(acc + bias) -> H (BF16)
 //   kEpiOut     acc + bias -> C (FP32), the columns n < Nv
-//   kEpiWgrad   the K slice's partial into ws (split K; the slices are added in
-//               order by the kernel that uses the gradients)
 // Every mbarrier wait is
 // bounded: a wait that runs out drains the copies and products in flight (again
 // bounded), sets the error flag and frees the tensor memory.  (mlp.cu includes
@@ -43,12 +38,11 @@ constexpr int kGtThreads = 256;
 constexpr int kGtStages = 4;
 constexpr size_t kGtMaxSmem = (size_t)kGtStages * (kGtM + 256) * 64 * 2 + 128;
 
-enum { kEpiHidden = 0, kEpiOut = 1, kEpiWgrad = 2 };
+enum { kEpiHidden = 0, kEpiOut = 1 };
 
 struct TcGemm {
     int M, N, K;     // rows computed (tiles of 128), columns (a multiple of BN), reduction length
     int BN, KC;      // column tile (16..256, a multiple of 16), K chunk (16, 32 or 64)
-    int kSlice;      // K of one split (a multiple of KC); gridDim.z = ceil(K / kSlice)
     int Mv, Nv;      // rows and columns of the result that exist
     int mode;
     const float* bias;
@@ -56,7 +50,6 @@ struct TcGemm {
     long long ldc;
     bf16* Hb;         // BF16 result, row-major
     long long ldh;
-    float* ws;        // kEpiWgrad: ws[(z * Mv + m) * Nv + n]
     int* err;
 };
 
@@ -87,16 +80,13 @@ __device__ __forceinline__ void store_bf16x32(bf16* p, const float (&v)[32])
                        pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
 }
 
-// Tile (bx, by) of the product, K slice bz; `partial`: into the slice's part of ws.
-__device__ __forceinline__ void gemm_tile(const CUtensorMap* ta, const CUtensorMap* tb, const TcGemm& g, int bx, int by,
-                                          int bz, bool partial)
+__global__ void __launch_bounds__(kGtThreads, 1)
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const TcGemm g)
 {
     extern __shared__ __align__(1024) unsigned char gsm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = bx * kGtM, n0 = by * g.BN;
-    const int kBeg = bz * g.kSlice;
-    const int kEnd = min(g.K, kBeg + g.kSlice);
-    const int nch = (kEnd - kBeg) / g.KC;
+    const int m0 = blockIdx.x * kGtM, n0 = blockIdx.y * g.BN;
+    const int nch = g.K / g.KC;
     const int S = nch < kGtStages ? nch : kGtStages;
     const uint32_t aBytes = (uint32_t)(kGtM * g.KC * 2), stBytes = aBytes + (uint32_t)(g.BN * g.KC * 2);
     uint64_t* bars = reinterpret_cast<uint64_t*>(gsm + (size_t)kGtStages * stBytes);  // full[4], done
@@ -131,10 +121,10 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap* ta, const CUtensorM
             const uint32_t par = (uint32_t)(pass & 1);
             for (int j = 0; j < cn; ++j) {
                 const uint32_t fb = smem_u32(&bars[j]);
-                const int kg = (kBeg + (c0 + j) * g.KC) >> 3;
+                const int kg = ((c0 + j) * g.KC) >> 3;
                 mbar_expect_tx(fb, stBytes);
-                tma_load4(base + (uint32_t)j * stBytes, ta, 0, 0, m0 >> 3, kg, fb);
-                tma_load4(base + (uint32_t)j * stBytes + aBytes, tb, 0, 0, n0 >> 3, kg, fb);
+                tma_load4(base + (uint32_t)j * stBytes, &ta, 0, 0, m0 >> 3, kg, fb);
+                tma_load4(base + (uint32_t)j * stBytes + aBytes, &tb, 0, 0, n0 >> 3, kg, fb);
             }
             int j = 0;
             for (; j < cn; ++j) {
@@ -178,21 +168,11 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap* ta, const CUtensorM
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = silu(v[j] + g.bias[nb + j]);
                 if (rv) store_bf16x32(g.Hb + row * g.ldh + nb, v);
-            } else if (g.mode == kEpiOut) {
+            } else {  // kEpiOut
                 if (rv)
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (nb + j < g.Nv) g.C[row * g.ldc + nb + j] = v[j] + g.bias[nb + j];
-            } else if (rv) {  // kEpiWgrad
-                float* dst = partial ? g.ws + ((long long)bz * g.Mv + row) * g.Nv : g.C + row * g.ldc;
-                const long long ld = partial ? g.Nv : g.ldc;
-                if (nb + 32 <= g.Nv && (ld & 3) == 0 && ((uintptr_t)dst & 15) == 0) {
-                    store_f32x32(dst + nb, v);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (nb + j < g.Nv) dst[nb + j] = v[j];
-                }
             }
         }
     }
@@ -202,12 +182,6 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap* ta, const CUtensorM
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     if (bad && tid == 0) atomicExch(g.err, 1);
-}
-
-__global__ void __launch_bounds__(kGtThreads, 1)
-    gemm_tc_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, const TcGemm g)
-{
-    gemm_tile(&ta, &tb, g, blockIdx.x, blockIdx.y, blockIdx.z, false);
 }
 
 // ---- host side -------------------------------------------------------------
@@ -261,7 +235,7 @@ cudaError_t gemm_tc(const CUtensorMap& ta, const CUtensorMap& tb, const TcGemm& 
 {
     if (g.M <= 0 || g.Mv <= 0) return cudaSuccess;
     if (g.BN < 16 || g.BN > 256 || g.BN % 16 || g.N % g.BN || (g.KC != 16 && g.KC != 32 && g.KC != 64) ||
-        g.K <= 0 || g.K % g.KC || g.kSlice != g.K || g.Nv > g.N || (g.mode == kEpiHidden && g.BN % 32))
+        g.K <= 0 || g.K % g.KC || g.Nv > g.N || (g.mode == kEpiHidden && g.BN % 32))
         return cudaErrorInvalidValue;
     const dim3 grid((unsigned)((g.M + kGtM - 1) / kGtM), (unsigned)(g.N / g.BN), 1);
     const size_t smem = (size_t)kGtStages * (kGtM + g.BN) * g.KC * 2 + 64;

@@ -12,16 +12,17 @@
 //   5, 6   dZ(l+1) W(l+1), l = 2, 1 256  256  dZl = acc * SiLU'(zl)
 //
 // Every stage's result is the next one's A operand and stays in shared memory; the
-// next weights are copied while the epilogue runs.  What leaves the CTA are the
-// operands of the weight gradients (X^T, H^T, dOut^T, dZ^T in BF16, zeros for the
-// rows past the minibatch), the FP32 dOut and dZ for the bias gradients, transposed
-// too (a warp stores a column of 32 rows at once), and z, which the same threads
-// read back (stored in their own order).
+// next weights are copied while the epilogue runs.  What leaves the CTA are those A
+// operands as they lie (X, H, dOut, dZ in BF16, by bulk copies while the products
+// run) -- the weight gradients read them back as MN-major operands, so nothing is
+// transposed --, the FP32 dOut and dZ for the bias gradients, transposed (a warp
+// stores a column of 32 rows at once), and z, which the same threads read back
+// (stored in their own order).
 //
 // Before, the step's chain was eleven launches of 6 to 15 us -- gather, four products,
 // loss, three products, each with its own descriptor fetch, tensor-memory allocation
 // and round trip through L2 -- 147 us a step with the weight gradients beside it, in
-// which the tensor pipe was busy for 5 %.  As three kernels: 89 us.
+// which the tensor pipe was busy for 5 %.  As three kernels: 72 us.
 
 // The weights in the operand layout (tc_off), in the order of the stages.
 constexpr uint32_t kPkW1 = 0;
@@ -34,6 +35,31 @@ constexpr uint32_t kPkW2T = kPkW3T + kHid * kHid * 2;
 constexpr uint32_t kPkBytes = kPkW2T + kHid * kHid * 2;
 
 constexpr int kStepStages = 7;
+constexpr int kMaxSplit = 16;  // K slices of a weight gradient
+
+// A tile's A operands (128 rows, layout tc_off(128, r, k)) in global memory.
+constexpr uint32_t kOpX = 0;
+constexpr uint32_t kOpH1 = kOpX + kTcM * kIn * 2;
+constexpr uint32_t kOpH2 = kOpH1 + kTcABytes;
+constexpr uint32_t kOpH3 = kOpH2 + kTcABytes;
+constexpr uint32_t kOpDOut = kOpH3 + kTcABytes;   // 32 columns
+constexpr uint32_t kOpDZ3 = kOpDOut + kTcM * kDOutPitch * 2;
+constexpr uint32_t kOpDZ2 = kOpDZ3 + kTcABytes;
+constexpr uint32_t kOpDZ1 = kOpDZ2 + kTcABytes;
+constexpr uint32_t kOpTile = kOpDZ1 + kTcABytes;
+constexpr uint32_t kOpGroup = kTcM * 16;          // 8 columns of an operand
+
+// Contiguous shared -> global bulk copy (16-byte aligned, a multiple of 16 bytes),
+// in this thread's next bulk group.
+__device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 constexpr int kGradRows = kOut + 3 * kHid;  // rows of StepArgs::gradT: dOut, dZ3, dZ2, dZ1
 
 struct StepArgs {
@@ -48,8 +74,8 @@ struct StepArgs {
     float fs, wLle;
     const unsigned char* wp;
     const float* params;
-    bf16 *xT, *h1T, *h2T, *h3T, *dOutT, *dz3T, *dz2T, *dz1T;
-    long long ld;          // pitch of the transposed outputs
+    unsigned char* ops;    // [tiles][kOpTile]: the tile's A operands, in stage order
+    long long ld;          // pitch of gradT
     float4* z;             // [3][tiles][16][512]
     float* gradT;          // [kGradRows][ld]
     float* out;            // optional: raw outputs, pitch kOut
@@ -143,14 +169,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
         const bool ok = mbar_wait(mbar, mph);
         mph ^= 1;
         tc_fence_after();
+        if (tid == 0) bulk_wait_read();  // the A operand has been copied out: its buffer may be written
         return !__syncthreads_or(!ok);
     };
-    // tensor-memory reads and A writes before the next products
-    auto handoff = [&]() {
+    // tensor-memory reads and A writes before the next products and the copy of the
+    // A operand to its place in the tile's operands
+    unsigned char* const ops = S.ops + (long long)blockIdx.x * kOpTile;
+    auto handoff = [&](uint32_t op, uint32_t bytes) {
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
+        if (tid == 0) {
+            bulk_s2g(ops + op, aAddr, bytes);
+            bulk_commit();
+        }
     };
     // 32 values of this thread's row as 32 columns of the next A operand
     auto to_operand = [&](int col0, const float (&v)[32]) {
@@ -162,11 +195,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
             *reinterpret_cast<uint4*>(A + tc_off(kTcM, row, col0 + 8 * i)) =
                 make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
     };
-    auto to_transposed = [&](bf16* T, int col0, const float (&v)[32]) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) T[(long long)(col0 + j) * S.ld + r] = __float2bfloat16_rn(rv ? v[j] : 0.0f);
-    };
-
     fetch(0);
     {
         // the minibatch row and its encoding: column quarter `part` of the inputs
@@ -190,14 +218,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
             *reinterpret_cast<uint4*>(A + tc_off(kTcM, row, 8 * j)) =
                 make_uint4(pack_bf16x2(e[0], e[1]), pack_bf16x2(e[2], e[3]), pack_bf16x2(e[4], e[5]),
                            pack_bf16x2(e[6], e[7]));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) S.xT[(long long)(8 * j + i) * S.ld + r] = __float2bfloat16_rn(e[i]);
         }
     }
-    handoff();
+    handoff(kOpX, kTcM * kIn * 2);
 
-    bf16* const hT[3] = {S.h1T, S.h2T, S.h3T};
-    bf16* const dzT[3] = {S.dz3T, S.dz2T, S.dz1T};
+    const uint32_t opOff[kStepStages] = {kOpH1, kOpH2, kOpH3, kOpDOut, kOpDZ3, kOpDZ2, kOpDZ1};
     const float* const bias[3] = {S.params + kB1, S.params + kB2, S.params + kB3};
     bool bad = false;
     for (int s = 0; s < kStepStages; ++s) {
@@ -221,7 +246,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
                 to_operand(col0, v);
-                to_transposed(hT[s], col0, v);
             }
         } else if (s == 3) {
             if (part == 0) {
@@ -254,8 +278,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
                 }
                 to_operand(0, d);
 #pragma unroll
-                for (int c = 0; c < kOut; ++c) S.dOutT[(long long)c * S.ld + r] = __float2bfloat16_rn(d[c]);
-#pragma unroll
                 for (int m = 16; m > 0; m >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, m);
                 if (lane == 0) atomicAdd(S.loss, loss);
             }
@@ -279,12 +301,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
                 if (rv)
 #pragma unroll
                     for (int j = 0; j < 32; ++j) gt[(long long)(col0 + j) * S.ld] = v[j];
-                if (l < 2) to_operand(col0, v);
-                to_transposed(dzT[l], col0, v);
+                to_operand(col0, v);
             }
         }
-        handoff();
+        handoff(opOff[s], s == 3 ? kTcM * kDOutPitch * 2 : kTcABytes);
     }
+    if (tid == 0) bulk_wait();
     if (bad && tid == 0) mbar_wait(wbar, wph ^ 1);  // the weights in flight, again bounded
     tc_fence_before();
     __syncthreads();
@@ -295,22 +317,124 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_step_kernel(const StepArgs 
 }
 
 // The weight gradients of all four layers, dW = dZ^T H over the minibatch, as one
-// launch: the CTAs of the four split-K products (gemm_tile, mlp_gemm_tc.cuh) side by
-// side, partials to each layer's region of ws.
-struct WgradGroup {
-    CUtensorMap a[4], b[4];
-    TcGemm g[4];
-    int nx[4], ny[4];
-    int first[5];  // first CTA of each product
+// launch: tiles of 128 rows and the whole width of the four products side by side,
+// split over K (the minibatch rows), partials to each layer's region of ws.  Seven
+// tiles, so that sixteen slices are one wave; 128 x 128 tiles would be two.
+//
+// Both operands are columns of the step kernel's A operands, whose layout for K =
+// rows is MN-major without swizzle: 8 columns x 8 rows of 16-byte pieces, 128 bytes
+// to the next 8 rows (leading-dimension byte offset), kOpGroup to the next 8 columns
+// (stride-dimension byte offset).  128 columns of a tile's 128 rows are one
+// contiguous 32 KB copy.  (With the operands transposed in global memory and fetched
+// through tensor maps of 16-byte rows, a step of 4096 rows took 89 us instead of 72:
+// the transposed two-byte stores of the step kernel cost as much as the products.)
+struct WgradProduct {
+    uint32_t a, b;       // operands within a tile's operands
+    uint32_t aBytes;     // bytes of A's columns (up to 128 of them)
+    int M, N;            // result M x N (N 128 or 256)
+    int nx, first;       // row tiles, first CTA
+    float* ws;
+};
+struct WgradArgs {
+    WgradProduct p[4];
+    const unsigned char* ops;
+    int K, slice;        // rows (a multiple of 64) and rows of a slice (a multiple of 64)
+    int* err;
 };
 
-__global__ void __launch_bounds__(kGtThreads, 1) mlp_wgrad_kernel(const __grid_constant__ WgradGroup W)
+constexpr int kWgThreads = 256, kWgStages = 2;
+constexpr uint32_t kWgHalf = 16 * kOpGroup;      // 128 columns of a tile: 32 KB
+constexpr uint32_t kWgStage = 3 * kWgHalf;       // A, and B of up to 256 columns
+constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 64;
+
+__global__ void __launch_bounds__(kWgThreads, 1) mlp_wgrad_kernel(const WgradArgs W)
 {
-    const int cta = (int)blockIdx.x;
+    extern __shared__ __align__(1024) unsigned char tsm[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tsm + (size_t)kWgStages * kWgStage);  // full[], done
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + kWgStages + 1);
+    int* flag = reinterpret_cast<int*>(slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int l = 0;
-    while (l < 3 && cta >= W.first[l + 1]) ++l;
-    const int i = cta - W.first[l];
-    gemm_tile(&W.a[l], &W.b[l], W.g[l], i % W.nx[l], (i / W.nx[l]) % W.ny[l], i / (W.nx[l] * W.ny[l]), true);
+    while (l < 3 && (int)blockIdx.x >= W.p[l + 1].first) ++l;
+    const WgradProduct& P = W.p[l];
+    const int i = (int)blockIdx.x - P.first;
+    const int bx = i % P.nx, bz = i / P.nx;
+    const int k0 = bz * W.slice, k1 = min(W.K, k0 + W.slice);
+    const int t0 = k0 / kTcM, nt = (k1 + kTcM - 1) / kTcM - t0;
+    const uint32_t base = smem_u32(tsm), doneBar = smem_u32(&bars[kWgStages]);
+
+    if (tid == 0) {
+        for (int j = 0; j <= kWgStages; ++j) mbar_init(smem_u32(&bars[j]), 1);
+        *flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
+                     "r"(256u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *slot;
+
+    if (tid == 0) {
+        const uint32_t bBytes = (uint32_t)(P.N / 8) * kOpGroup;
+        const uint32_t idesc = tc_idesc(kTcM, P.N) | (1u << 15) | (1u << 16);  // both operands MN-major
+        bool ok = true, first = true;
+        for (int c = 0, pass = 0; c < nt && ok; c += kWgStages, ++pass) {
+            const int cn = min(kWgStages, nt - c);
+            const uint32_t par = (uint32_t)(pass & 1);
+            for (int j = 0; j < cn; ++j) {
+                const uint32_t fb = smem_u32(&bars[j]), at = base + (uint32_t)j * kWgStage;
+                const unsigned char* tile = W.ops + (long long)(t0 + c + j) * kOpTile;
+                mbar_expect_tx(fb, P.aBytes + bBytes);
+                bulk_g2s(at, tile + P.a + (uint32_t)bx * kWgHalf, P.aBytes, fb);
+                bulk_g2s(at + kWgHalf, tile + P.b, bBytes, fb);
+            }
+            int j = 0;
+            for (; j < cn; ++j) {
+                if (!mbar_wait(smem_u32(&bars[j]), par)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t at = base + (uint32_t)j * kWgStage;
+                const int r0 = (t0 + c + j) * kTcM;
+                for (int r = max(r0, k0); r < min(r0 + kTcM, k1); r += 16) {
+                    const uint32_t off = (uint32_t)((r - r0) / 8) * 128u;
+                    tc_mma(tmem, tc_desc(at + off, 128, kOpGroup), tc_desc(at + kWgHalf + off, 128, kOpGroup), idesc,
+                           first ? 0u : 1u);
+                    first = false;
+                }
+            }
+            // on a failed wait: let the copies still in flight land (bounded)
+            if (!ok)
+                for (int m = j; m < cn; ++m) mbar_wait(smem_u32(&bars[m]), par);
+            tc_commit(doneBar);
+            if (!mbar_wait(doneBar, par)) ok = false;  // the products have read every stage
+        }
+        if (!ok) *flag = 1;
+    }
+    __syncthreads();
+    tc_fence_after();
+    const bool bad = *flag != 0;
+    if (!bad && nt > 0) {
+        const int q = warp & 3, row = bx * kTcM + 32 * q + lane;
+        const uint32_t lb = tmem + ((uint32_t)(32 * q) << 16);
+        for (int ch = warp >> 2; ch < P.N / 32; ch += 2) {
+            float v[32];
+            tmem_ld32(lb + (uint32_t)(ch * 32), v);
+            if (row < P.M) store_f32x32(P.ws + ((long long)bz * P.M + row) * P.N + ch * 32, v);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    if (bad && tid == 0) atomicExch(W.err, 1);
 }
 
 // Where the gradient of a parameter comes from: the slices of its layer's split-K
@@ -333,8 +457,13 @@ __device__ __forceinline__ float weight_grad(const GradSource& G, long long i)
     else if (i < kB3) { l = 1; at = i - kW3; mn = (long long)kHid * kHid; }
     else { l = 0; at = i - kW4; mn = (long long)kOut * kHid; }
     const float* p = G.ws + l * G.wsLayer + at;
+    float v[kMaxSplit];  // the loads together, the additions in order
+#pragma unroll
+    for (int z = 0; z < kMaxSplit; ++z) v[z] = z < G.splits ? p[z * mn] : 0.f;
     float acc = 0.f;
-    for (int z = 0; z < G.splits; ++z) acc += p[z * mn];
+#pragma unroll
+    for (int z = 0; z < kMaxSplit; ++z)
+        if (z < G.splits) acc += v[z];
     return acc;
 }
 
@@ -357,7 +486,15 @@ __device__ __forceinline__ float bias_grad(const GradSource& G, int c, int lane)
 {
     const float* g = G.gradT + (long long)c * G.ld;
     float s = 0.f;
-    for (int m = lane; m < G.n; m += 32) s += g[m];
+    int m = lane;
+    for (; m + 7 * 32 < G.n; m += 8 * 32) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = g[m + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; m < G.n; m += 32) s += g[m];
     float t = 0.f;
 #pragma unroll
     for (int r = 0; r < 32; ++r) t += __shfl_sync(0xffffffffu, s, r);
