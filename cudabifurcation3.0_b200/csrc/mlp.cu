@@ -267,8 +267,9 @@ struct Mlp {
     float* yl = nullptr;
     int* yc = nullptr;
     unsigned char* ops = nullptr;  // the step kernel's operands, tile by tile
-    float* z = nullptr;        // pre-activations, in the step kernel's own order
     float* out = nullptr;
+    float* z = nullptr;        // pre-activations, in the one-CTA step kernel's own order
+    int clusters = 0;          // clusters of the step kernel that are resident at once
     float* gradT = nullptr;    // FP32 dOut, dZ3, dZ2, dZ1, transposed, for the bias gradients
     float* loss = nullptr;
     float* ws = nullptr;      // split-K partials, one region per weight gradient
@@ -363,11 +364,16 @@ cudaError_t step_products(Mlp& m, StepArgs a, cudaStream_t s, GradSource* src)
     a.params = m.params;
     a.ops = m.ops;
     a.ld = m.Ba;
-    a.z = (float4*)m.z;
     a.gradT = m.gradT;
     a.loss = m.loss;
     a.err = m.gemmErr;
-    mlp_step_kernel<<<(unsigned)tiles, kTcThreads, kTcSmem, s>>>(a);
+    // one wave of clusters, or one CTA a tile (both measured in mlp_step.cuh)
+    if (tiles <= m.clusters) {
+        mlp_step_cluster_kernel<<<(unsigned)tiles * kStC, kTcThreads, kStSmem, s>>>(a);
+    } else {
+        a.z = (float4*)m.z;
+        mlp_step_kernel<<<(unsigned)tiles, kTcThreads, kTcSmem, s>>>(a);
+    }
     note_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -433,7 +439,7 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
     A_(params, kNumParams); A_(grads, kNumParams); A_(m1, kNumParams); A_(m2, kNumParams);
     A_(tw, kNumSlots * kSlot); A_(wp, (long long)kPkBytes);
     A_(xraw, Ba * kRaw); A_(yl, Ba); A_(yc, Ba);
-    A_(ops, Ba / kTcM * kOpTile); A_(z, 3 * Ba * kHid);
+    A_(ops, Ba / kTcM * kOpTile);
     A_(out, Ba * kOut); A_(gradT, kGradRows * Ba);
     A_(loss, 1); A_(step, 1); A_(finished, 1); A_(gemmErr, 1);
     A_(ws, 4ll * kMaxSplit * kHid * kHid);
@@ -454,6 +460,22 @@ cbf_status mlp_alloc(cbf_mlp* m, int B)
         e = cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_step_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStSmem);
+    if (e == cudaSuccess) {
+        cudaLaunchConfig_t c = {};
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kStC;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        c.gridDim = dim3(kStC);
+        c.blockDim = dim3(kTcThreads);
+        c.dynamicSmemBytes = kStSmem;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        e = cudaOccupancyMaxActiveClusters(&m->clusters, mlp_step_cluster_kernel, &c);
+    }
+    if (e == cudaSuccess && Ba / kTcM > m->clusters) e = alloc_zero(&m->z, 3 * Ba * kHid);
     if (e != cudaSuccess) return report_cuda_error(e, "surrogate network tensor maps");
     return CBF_OK;
 }
