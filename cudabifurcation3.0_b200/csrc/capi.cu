@@ -414,7 +414,7 @@ cbf_status run_lowered(const DevJob& d, void* d_out, void* d_aux, cudaStream_t s
 // and laid out in the caller's rows.  What lies past a row's count is unspecified
 // and not copied: a 1000-point diagram of 25 000 slots a row holds 0.7 MB of peaks
 // in 200 MB (its copy took 45 of 63 ms).  *done is false where more than half of
-// the slots are filled, or host memory for the pieces is short; the whole rows are
+// the slots are filled, or memory for the pieces is short; the whole rows are
 // copied then.
 cudaError_t copy_packed_peaks(const DevJob& d, const double* d_peaks, const int* d_counts, const int* counts,
                               double* out, cudaStream_t s, bool* done)
@@ -432,12 +432,16 @@ cudaError_t copy_packed_peaks(const DevJob& d, const double* d_peaks, const int*
     if (2 * total > n * cap) return cudaSuccess;
     std::unique_ptr<double[]> host(new (std::nothrow) double[(size_t)total + 1]);
     if (!host) return cudaSuccess;
-    *done = true;
-    if (total == 0) return cudaSuccess;
     char* mem = nullptr;
     const size_t offBytes = (size_t)n * sizeof(long long);
-    cudaError_t e = cudaMallocAsync((void**)&mem, offBytes + (size_t)total * sizeof(double), s);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (total > 0) e = cudaMallocAsync((void**)&mem, offBytes + (size_t)total * sizeof(double), s);
+    if (e == cudaErrorMemoryAllocation) {  // no room beside the rows: they are copied whole
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    *done = true;
+    if (total == 0 || e != cudaSuccess) return e;
     auto* d_packed = (double*)(mem + offBytes);
     e = cudaMemcpyAsync(mem, offset.get(), offBytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = launch_pack_peaks(d_peaks, d_counts, (const long long*)mem, n, d.peakCap, d_packed, s);
