@@ -30,8 +30,8 @@
 // What bounds it is the chain of seven stages, not a unit: of the 7400 cycles of a
 // middle stage, 2700 are the exchange (48 KB in and out of each SM), 1600 the sixteen
 // products, 1500 the epilogue's arithmetic (sent group by group, it overlaps the
-// exchange) and the rest waits.  A step of 4096 rows takes 55 us, of which this kernel
-// is about 27; with one CTA for a tile (below) 72 us; as eleven launches -- gather,
+// exchange) and the rest waits.  A step of 4096 rows takes 53 us, of which this kernel
+// is about 27; with one CTA for a tile (below) 17 us more; as eleven launches -- gather,
 // four products, loss, three products, each with its own descriptor fetch,
 // tensor-memory allocation and round trip through L2 -- 143 us.
 
@@ -781,20 +781,22 @@ __device__ __forceinline__ long long bias_param(int c)
 }
 
 // A warp's sum of column c: lane t adds rows t, t + 32, ..., then the 32 partial
-// sums are added in order.
+// sums are added in order.  Sixteen loads in flight, and the bias warps in the first
+// blocks of the grid: the columns of 4096 rows are the longest chain of the kernel
+// (a step 55 -> 53 us against eight loads and last blocks; thirty-two take too many
+// registers for the grid to be resident).
 __device__ __forceinline__ float bias_grad(const GradSource& G, int c, int lane)
 {
     const float* g = G.gradT + (long long)c * G.ld;
     float s = 0.f;
-    int m = lane;
-    for (; m + 7 * 32 < G.n; m += 8 * 32) {
-        float v[8];
+    for (int m = lane; m < G.n; m += 16 * 32) {
+        float v[16];  // the loads together, the additions in order
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = g[m + 32 * u];
+        for (int u = 0; u < 16; ++u) v[u] = m + 32 * u < G.n ? g[m + 32 * u] : 0.f;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) s += v[u];
+        for (int u = 0; u < 16; ++u)
+            if (m + 32 * u < G.n) s += v[u];
     }
-    for (; m < G.n; m += 32) s += g[m];
     float t = 0.f;
 #pragma unroll
     for (int r = 0; r < 32; ++r) t += __shfl_sync(0xffffffffu, s, r);
@@ -805,19 +807,20 @@ constexpr int kParamThreads = 256;
 constexpr int kParamBlocks = (int)((kNumParams + kParamThreads - 1) / kParamThreads);
 constexpr int kBiasBlocks = (kGradRows + kParamThreads / 32 - 1) / (kParamThreads / 32);
 
-// use(i, gradient) for every parameter: a thread per weight, a warp per bias.
+// use(i, gradient) for every parameter: a warp per bias (first: they take longest),
+// a thread per weight.
 template <class Use>
 __device__ __forceinline__ void each_gradient(const GradSource& G, Use use)
 {
-    if ((int)blockIdx.x < kParamBlocks) {
-        const long long i = (long long)blockIdx.x * kParamThreads + threadIdx.x;
-        if (i < kNumParams && !is_bias(i)) use(i, weight_grad(G, i));
-    } else {
-        const int c = ((int)blockIdx.x - kParamBlocks) * (kParamThreads / 32) + (int)(threadIdx.x >> 5);
+    if ((int)blockIdx.x < kBiasBlocks) {
+        const int c = (int)blockIdx.x * (kParamThreads / 32) + (int)(threadIdx.x >> 5);
         if (c < kGradRows) {
             const float g = bias_grad(G, c, threadIdx.x & 31);
             if ((threadIdx.x & 31) == 0) use(bias_param(c), g);
         }
+    } else {
+        const long long i = (long long)((int)blockIdx.x - kBiasBlocks) * kParamThreads + threadIdx.x;
+        if (i < kNumParams && !is_bias(i)) use(i, weight_grad(G, i));
     }
 }
 
