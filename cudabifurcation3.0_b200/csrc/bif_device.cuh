@@ -90,13 +90,13 @@ struct StateOf {
 // FP64 comparisons, the divergence test, the state machine's branches) cost more
 // than the step: 103 ms for 40 000 samples x 1024^2 Lorenz points where 100 000
 // bare steps take 72 ms.  So samples are taken in blocks of kRing: per sample one
-// FP64 subtraction whose sign bit (d[i] above d[i-1]) is shifted into a mask, one
-// shared-memory store and half a three-input maximum against the threshold; the
-// block's peaks then follow from the mask's few candidates (44 ms; the 1024^2
-// DBSCAN map 256 -> 205 ms, a ragged batch 112 -> 86 ms).  A block in which a
-// sample may have reached the divergence threshold or is no number is repeated
-// from its first state with the exact per-sample code; so is the end of the
-// record.
+// FP64 subtraction whose sign bit (d[i] above d[i-1]) is shifted into a mask
+// (RiseMask), one shared-memory store, half a three-input minimum for the mask and
+// half a three-input maximum against the threshold; the block's peaks then follow
+// from the mask's few candidates (44 ms; the 1024^2 DBSCAN map 256 -> 205 ms, a
+// ragged batch 112 -> 86 ms).  A block in which a sample may have reached the
+// divergence threshold or is no number is repeated from its first state with the
+// exact per-sample code; so is the end of the record.
 template <class S, int WV, bool PRE1, bool WITH_INTERVALS, class Hook>
 __device__ __forceinline__ bool record_loop(const RecordSpec& R, double (&x)[S::DIM], const typename S::Coef& c,
                                             PeakStream& ps, double* ring, double* pk, double* iv, Hook& hook)
@@ -120,21 +120,22 @@ __device__ __forceinline__ bool record_loop(const RecordSpec& R, double (&x)[S::
             for (int i = 0; i < D; ++i) x0[i] = x[i];
             HiTrack tr;
             tr.init();
-            unsigned up = 0;
+            RiseMask<kRing> rises;
+            rises.init();
             double p = ps.prev1;
             ring[0] = p;
 #pragma unroll (D == 5 ? 1 : 2)
             for (int i = 0; i < kRing; i += 2) {
                 const double a = next();
-                up = __funnelshift_l((unsigned)__double2hiint(p - a), up, 1);
+                const int up = rises.add(p, a);
                 ring[32 * i + 32] = a;
                 p = next();
-                up = __funnelshift_l((unsigned)__double2hiint(a - p), up, 1);
+                rises.seen(up, rises.add(a, p));
                 ring[32 * i + 64] = p;
                 tr.add2(a, p);
             }
             if (!tr.maybe(R.hiT)) {
-                ps.push_block<kRing, WITH_INTERVALS>(up, t, kRing, p, ring, pk, iv, R.cap, hook);
+                ps.push_block<kRing, WITH_INTERVALS>(rises.mask(kRing, ring), t, kRing, p, ring, pk, iv, R.cap, hook);
                 t += kRing;
                 continue;
             }

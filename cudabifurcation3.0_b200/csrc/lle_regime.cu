@@ -107,7 +107,8 @@ __device__ __forceinline__ void window_loop(const WindowSpec& W, WindowState<S>&
                 HiTrack tr, num;
                 tr.init();
                 num.init();
-                unsigned up = 0;
+                RiseMask<kRing> rises;
+                rises.init();
                 double p = ps.prev1;
                 ring[0] = p;
 #pragma unroll (D == 5 ? 1 : 4)
@@ -115,17 +116,18 @@ __device__ __forceinline__ void window_loop(const WindowSpec& W, WindowState<S>&
                     S::step(x, c);
                     S::step(y, c);
                     const double v = sample_of<S, WV>(x, W.wv, c);
-                    up = __funnelshift_l((unsigned)__double2hiint(p - v), up, 1);
+                    const int up = rises.add(p, v);
+                    rises.seen(up, up);
                     ring[32 * k] = v;
                     p = v;
                     tr.add2(x[0], y[0]);
                     if (WV != 0) num.add1(v);
                 }
-                up <<= kRing - m;
                 done = !tr.maybe(W.hiT) && (WV == 0 || !num.maybe(0x7f800000u));
                 if (done) {
                     const int fed = max(0, min(m, steps - 1 - t));  // samples t+1 .. t+fed are in the window
                     if (fed > 0) {
+                        const unsigned up = rises.mask(m, ring);
                         if (W.amplitude) {
                             // a sample is a local extreme where it rose and its
                             // successor does not, or the other way round

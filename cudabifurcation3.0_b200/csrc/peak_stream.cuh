@@ -4,6 +4,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
+#include <string.h>
 
 namespace cbf {
 namespace {
@@ -30,6 +32,60 @@ __host__ __device__ __forceinline__ int highest_bit(unsigned v)
     return 31 - __builtin_clz(v);
 #endif
 }
+
+// The rises of a block of K samples, collected as they come: bit K-1-i is set where
+// sample i + 1 of the block is above sample i, sample 0 being the one before the
+// block.  The sign of the difference p - v says so -- a subtraction of different
+// numbers is never 0, and 0 has no sign bit -- with one exception: (-0) - (+0) is -0.
+// A difference whose high word is the sign alone is that, or a negative number below
+// 2^-1042, so the smallest high word tells whether the signs can be trusted; where
+// they cannot, the block's samples are compared.  The minimum takes two samples an
+// instruction; it costs the 1024^2 DBSCAN map 1 of 147 ms (without it 146, with wrong
+// peaks from trajectories that start on -0).
+template <int K>
+struct RiseMask {
+    unsigned signs;
+    int least;
+
+    __host__ __device__ __forceinline__ void init()
+    {
+        signs = 0;
+        least = INT_MAX;
+    }
+    // Sample v after sample p: the difference's high word, to be given to seen().
+    __host__ __device__ __forceinline__ int add(double p, double v)
+    {
+        const double d = p - v;
+#ifdef __CUDA_ARCH__
+        const int hi = __double2hiint(d);
+        signs = __funnelshift_l((unsigned)hi, signs, 1);
+#else
+        long long b;
+        memcpy(&b, &d, sizeof(b));
+        const int hi = (int)(b >> 32);
+        signs = signs << 1 | (unsigned)hi >> 31;
+#endif
+        return hi;
+    }
+    __host__ __device__ __forceinline__ void seen(int hi1, int hi2)
+    {
+#ifdef __CUDA_ARCH__
+        least = __vimin3_s32(least, hi1, hi2);
+#else
+        least = hi1 < least ? hi1 : least;
+        least = hi2 < least ? hi2 : least;
+#endif
+    }
+    // The mask of the first m samples after ring[0], all of them added and seen.
+    __host__ __device__ __forceinline__ unsigned mask(int m, const double* ring) const
+    {
+        if (least != INT_MIN) return signs << (K - m);
+        unsigned up = 0;
+#pragma unroll 1
+        for (int i = 0; i < m; ++i) up = up << 1 | (ring[32 * i + 32] > ring[32 * i] ? 1u : 0u);
+        return up << (K - m);
+    }
+};
 
 struct NoPeakHook {
     __host__ __device__ __forceinline__ void operator()(double, int) const {}
@@ -127,8 +183,7 @@ struct PeakStream {
 
     // m <= K samples at once: the samples of times t+1 .. t+m (prev1 is time t's),
     // all of them numbers, in ring[32 * 1] .. ring[32 * m] with time t's in ring[0];
-    // bit K-1-i of `up`: sample t+1+i is above its predecessor.  Equal to m calls
-    // of push().  A candidate arrival is one that does not rise after one that
+    // `up`: the block's rises (RiseMask).  Equal to m calls of push().  A candidate arrival is one that does not rise after one that
     // did.  The SKIP after a peak is implied -- a sample right after a descent
     // cannot be such an arrival -- so only plateaus need the state.
     template <int K, bool WITH_INTERVALS, class Hook>
