@@ -348,19 +348,23 @@ def make_job(*, task, system, nPts, ranges, idxMut, ic, values, h, tMax=0.0, tra
     return j
 
 
+_OWN_MAPPING = 32 << 20  # glibc maps every larger block by itself, whatever was freed before
+
+
 def _peak_rows(n: int, cap: int) -> np.ndarray:
-    """Zeros of shape (n, cap) for peak rows, of which a few slots are written: small
-    pages, so that a written row costs its own page and not the zeroing of the 2 MB
-    around it (numpy asks for huge pages; 200 MB of rows took 20 ms)."""
-    size = 8 * n * cap
-    if size < 1 << 21 or not hasattr(mmap, "MADV_NOHUGEPAGE"):
+    """Zeros of shape (n, cap) for peak rows, of which a few slots are written: fresh
+    small pages, so that a written row costs its own page and not the zeroing of the
+    2 MB around it (numpy asks for huge pages: 200 MB of rows took 20 ms) or of memory
+    used before.  An array like any other: private, and it owns its data."""
+    if 8 * n * cap < 1 << 21 or not hasattr(mmap, "MADV_NOHUGEPAGE"):
         return np.zeros((n, cap), np.float64)
-    pages = mmap.mmap(-1, size)
-    try:
-        pages.madvise(mmap.MADV_NOHUGEPAGE)
-    except OSError:  # a kernel without huge pages
-        pass
-    return np.frombuffer(pages, np.float64).reshape(n, cap)
+    rows = np.zeros(max(n * cap, _OWN_MAPPING // 8 + 1024), np.float64)
+    rows.resize((n, cap), refcheck=False)  # gives the rest of the mapping back
+    first = -(-rows.ctypes.data // mmap.PAGESIZE) * mmap.PAGESIZE
+    size = (rows.ctypes.data + rows.nbytes) // mmap.PAGESIZE * mmap.PAGESIZE - first
+    # only advice: refused by a kernel without huge pages
+    C.CDLL(None).madvise(C.c_void_p(first), C.c_size_t(size), C.c_int(mmap.MADV_NOHUGEPAGE))
+    return rows
 
 
 def run_host(job: Job):
