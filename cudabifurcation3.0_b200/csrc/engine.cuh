@@ -217,6 +217,13 @@ cudaError_t launch_ls_seeds(const DevJob& J, double* d_out, cudaStream_t s);
 cudaError_t launch_lle_regime(const DevJob& J, double* d_lle, int* d_class, cudaStream_t s);
 // Points of one wave of the surrogate map's recompute rounds on the current device.
 long long lle_regime_round_points(const DevJob& J);
+// Blocks of `bytes` of dynamic shared memory each that fit an SM's `perSm` bytes: a
+// block takes `reserved` bytes more, and whole units of 128 (what the occupancy
+// calculator counts: of 233 472 bytes, 45 568 a block are five blocks, 45 584 four).
+inline long long blocks_by_shared_memory(long long perSm, long long bytes, long long reserved)
+{
+    return perSm / ((bytes + reserved + 127) / 128 * 128);
+}
 // The LLE_REGIME kernel over a device point list (J.pointIndex) whose length
 // *nDev (at most maxPoints) a previous kernel wrote, with caller-provided
 // scratch of lle_regime_scratch_bytes(J); no allocation, no host

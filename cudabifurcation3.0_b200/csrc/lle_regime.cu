@@ -451,7 +451,7 @@ long long lle_regime_round_points(const DevJob& J)
         cudaDeviceGetAttribute(&perSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
         return 0;
-    const long long fit = perSm / (kRegWarps * words * (long long)sizeof(unsigned) + reserved);
+    const long long fit = blocks_by_shared_memory(perSm, kRegWarps * words * (long long)sizeof(unsigned), reserved);
     return (long long)sms * (fit < 6 ? fit : 6) * kRegThreads;
 }
 
