@@ -136,7 +136,8 @@ cbf_status launch_family(cbf_batch* b, int f, void* d_jobs, long long* d_end, in
 // One run: the error flag cleared, then every non-empty family's persistent
 // kernel; with two families the second runs on the side stream (fork/join by
 // events, which stream capture records as parallel branches), so its blocks
-// take the SMs the first family's blocks leave as its queue drains.
+// take the SMs the first family's blocks leave as its queue drains (blocks of the
+// peak family that find no tile left help the others and leave once that is idle).
 cbf_status launch_all(cbf_batch* b, cudaStream_t s)
 {
     cudaError_t e = cudaMemsetAsync(b->d_err, 0, sizeof(int), s);
