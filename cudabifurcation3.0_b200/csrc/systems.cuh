@@ -111,6 +111,10 @@ __host__ __device__ __forceinline__ double divide_maybe_zero(double a, double b)
 // before its dividend, but its reciprocal taken ahead the same way made a step
 // longer (32^2 points: 3.7 ms): the compiler's reciprocal is a branch that nothing
 // overlaps.
+// A dividend out of range is divided as written, but for one that is no number, whose
+// quotient is none either: the spectra of 32^2 points without a bound, a third of which
+// leave the numbers, take 18.6 ms (24.1 with those divided too, 21.6 with the
+// compiler's division alone).
 // Rounding to float by integer operations on the words instead of the conversions
 // there and back made a step shorter by itself but a full SM's steps longer: five
 // roundings are 30 integer operations at half rate, and the conversions have a
@@ -170,8 +174,8 @@ struct Memristive5 {
         if (!LITERAL) {
             const unsigned p2 = operand_place(n2), p3 = operand_place(n3);
             if ((p2 > p3 ? p2 : p3) >= c.span) {
-                x[2] = n2 / c.d2.b;
-                x[3] = n3 / c.d3.b;
+                if (n2 == n2) x[2] = n2 / c.d2.b;
+                if (n3 == n3) x[3] = n3 / c.d3.b;
             }
         }
         x[4] = y4 + h1 * (x[0]);
