@@ -68,7 +68,9 @@ __device__ __forceinline__ void renormalise(double (&x)[S::DIM], double (&y)[S::
 // (loopCalculateDiscreteModel, cudaLibrary.cu:55-74).  A function of its own, so
 // that its state does not shape the register use of the pair loop after it.
 // Before, the window ran the exact tests and the state machine on every step
-// (Chen 600^2, window a tenth of the record: 200 -> 185 ms, and 174 ms with the tile counter).
+// (Chen 600^2, window a tenth of the record: 200 -> 185 ms, and 174 ms with the tile
+// counter).  A single sample is no block: intervals of one step, Chen 100^2 with a
+// third of the record in the window, take 11.6 ms with the exact tests, 12.1 in blocks.
 template <class S, int WV>
 __device__ __forceinline__ void window_loop(const WindowSpec& W, WindowState<S>& st, const typename S::Coef& c,
                                             double* ring, double* pk, double* iv)
@@ -100,7 +102,7 @@ __device__ __forceinline__ void window_loop(const WindowSpec& W, WindowState<S>&
             const int m = min(kRing, W.nNT - i);
             i += m;
             bool done = false;
-            if (!fired && ax && ay) {
+            if (!fired && ax && ay && m > 1) {
                 double x0[D], y0[D];
                 copy_state<D>(x0, x);
                 copy_state<D>(y0, y);
