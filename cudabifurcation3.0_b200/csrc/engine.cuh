@@ -1,6 +1,5 @@
 // Internal definitions shared by the kernels and the C-ABI layer.
 #pragma once
-#include <limits.h>
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -106,11 +105,6 @@ __device__ __forceinline__ void setup_point(const DevJob& J, long long g, double
         }
         v[i] = t;
     }
-}
-
-__device__ __forceinline__ unsigned abs_hi(double v)
-{
-    return (unsigned)(__double_as_longlong(v) >> 32) & 0x7fffffffu;
 }
 
 // Conservative magnitude tracker of a stream of doubles against a threshold T:
