@@ -8,7 +8,8 @@
 // register count and occupancy); with both present the two kernels run
 // concurrently on forked streams:
 //   * every job is cut into tiles of 32 points (one warp: a lane per point; fewer
-//     points in a small batch of peak jobs, whose epilogues run one by one);
+//     points in a small batch of peak jobs, whose epilogues a warp runs one after
+//     the other, shared with the warps that find no tile left);
 //   * jobs are ordered by estimated cost per point, longest first, and a prefix
 //     table of tile counts maps a global tile number to (job, tile);
 //   * each warp takes the next tile number from a device counter (atomicAdd by
@@ -121,11 +122,16 @@ __device__ __forceinline__ int run_tile(const DevJob& J, void* out, int* aux, lo
 // WITH_M5: also dispatch the 5-D shipped model.  Its wider state raises the
 // register count of the whole kernel, so batches of 3-D systems use the
 // instantiation without it.
-// Four blocks of 128 threads per SM (128 registers) in both families: the FP64
+// Four blocks of 128 threads per SM (128 registers) in both families.  LLE: the FP64
 // chains issue best from an even number of warps per scheduler (see lle.cu; at six
-// blocks the LLE jobs of a 24-job mix took 30 ms, at four 24).  Peak jobs' epilogues
-// are shared by the warps that have run out of tiles (the same mix's peak jobs: 43
-// -> 35 ms; the two families side by side, two blocks per SM each, were no faster).
+// blocks the LLE jobs of a 24-job mix of 64^2 to 256^2 points took 30 ms, at four
+// 24).  Peaks: the same mix's peak jobs take 35.1 ms at four, 37.1 at six (80
+// registers) and 41.6 at eight (64 registers, 0.6 KB spilled); what a small mix waits
+// for is its last tiles, which go slower the more warps share an SM.  Where tiles are
+// many the order is another: 24 jobs of 300^2 to 500^2, 182, 164 and 173 ms; a mix of
+// 64 jobs, 27 million points, both families, 26.7 s at four and 25.4 at six.  The
+// peak jobs' shared epilogues took the small mix's from 43 to 35 ms (the two families
+// side by side, two blocks per SM each, were no faster).
 template <int FAM, bool WITH_M5>
 __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(
     const BatchJob* __restrict__ jobs, int nJobs, const long long* __restrict__ tileEnd,

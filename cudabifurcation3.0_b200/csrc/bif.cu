@@ -6,19 +6,22 @@
 // kdeCUDA (:356-441) or dbscanCUDA (:457-624) reduce each point.
 //
 // Here one fused kernel does all of it.  Each lane of a warp owns one point and
-// keeps the ODE state in registers; the recorded variable is never stored: a
-// streaming state machine reproduces peakFinder exactly (see PeakStream) and
-// only the peaks (and intervals) go to a per-warp scratch slice in HBM.  Then
-// the warp reduces its 32 points one after the other, cooperatively:
-//   KDE    -- lanes take 32 consecutive sample positions; each sums its kernel
-//             terms over the peaks in the reference's peak order (double sum of
-//             FP32 expf), so the sums are bit-identical; the plateau state
-//             machine then runs over the 32 sums via shuffles.
+// keeps the ODE state in registers; the recorded variable is never stored: blocks
+// of 16 samples feed a streaming state machine that reproduces peakFinder exactly
+// (record_loop, PeakStream), and only the peaks (and intervals) go to a per-warp
+// scratch slice in HBM.  Then a warp reduces one point at a time, cooperatively --
+// its own tile's, and when the tiles have run out other warps' (EpilogueShare):
+//   KDE    -- lanes take 32 consecutive sample positions; the signs of neighbouring
+//             sums are settled by FP32 sums with an error bound where those can
+//             decide, else by the reference's own sums (a double sum of FP32 expf in
+//             its peak order, bit-identical); the plateau state machine then runs
+//             over the signs (kde_warp).
 //   DBSCAN -- labels and the reference's neighbour "stack" become two bitsets
 //             in shared memory; the inner neighbour loop over k is a ballot
 //             (its iterations are independent in the reference), popcount
 //             updates the neighbour counter.
-// Results leave as one coalesced store per tile.
+// A point's result leaves as one 4-byte store when its epilogue ends (OSTROVSKY,
+// whose epilogues stay with their warp: one coalesced store per tile).
 //
 // Tiles are taken from a device counter: how long a point's epilogue takes
 // depends on its peaks, and a fixed assignment left the warps with few of them

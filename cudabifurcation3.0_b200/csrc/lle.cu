@@ -165,7 +165,7 @@ cudaError_t launch_variant(const DevJob& J, double* d_out, cudaStream_t s)
 //   7: 1 pt, 128 thr, no cap, unroll 8
 // Chen 1024^2, 50 000 transient steps and 100 000 pairs: shapes 1..7 take 173,
 // 181, 178, 178, 172, 180, 170 ms, 64 registers with unroll 2 (the default
-// before) 182, the default now 170 (lle map at full length: 908 -> 848 ms).
+// before) 182, the default now 170 (250 000 and 500 000, host arrays: 944 -> 857 ms).
 template <class S, bool IC>
 cudaError_t launch_lle_v(const DevJob& J, double* d_out, cudaStream_t s, int variant)
 {

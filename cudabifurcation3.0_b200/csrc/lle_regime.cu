@@ -11,9 +11,10 @@
 //      it has more than maxAmountOfPeaks peaks, or 15 or more clusters.
 // A window whose samples span less than regimeMinAmp is class 0 as well: an
 // equilibrium reached to FP64 precision can still wobble by an ulp and show
-// spurious peaks.  The window costs one peak-state update per step on top of the LLE; the
-// transient is shared.  This is the plain FP64 method that labels the surrogate's
-// training data and recomputes the points it cannot be trusted with.
+// spurious peaks.  On top of the LLE the window costs a few integer instructions and a
+// shared-memory store per step, and the peak states of a block's candidates
+// (window_loop); the transient is shared.  This is the plain FP64 method that labels
+// the surrogate's training data and recomputes the points it cannot be trusted with.
 #include "bif_device.cuh"
 #include "lle_device.cuh"
 

@@ -183,9 +183,10 @@ struct PeakStream {
 
     // m <= K samples at once: the samples of times t+1 .. t+m (prev1 is time t's),
     // all of them numbers, in ring[32 * 1] .. ring[32 * m] with time t's in ring[0];
-    // `up`: the block's rises (RiseMask).  Equal to m calls of push().  A candidate arrival is one that does not rise after one that
-    // did.  The SKIP after a peak is implied -- a sample right after a descent
-    // cannot be such an arrival -- so only plateaus need the state.
+    // `up`: the block's rises (RiseMask).  Equal to m calls of push().  A candidate
+    // arrival is one that does not rise after one that did.  The SKIP after a peak is
+    // implied -- a sample right after a descent cannot be such an arrival -- so only
+    // plateaus need the state.
     template <int K, bool WITH_INTERVALS, class Hook>
     __host__ __device__ __forceinline__ void push_block(unsigned up, int t, int m, double last, const double* ring,
                                                         double* pk, double* iv, int cap, Hook& hook)

@@ -105,12 +105,14 @@ __host__ __device__ __forceinline__ double divide_maybe_zero(double a, double b)
 //
 // Two of the three divisions have divisors of the parameters alone; those run as
 // above, with one look at both dividends' ranges (5 dependent FP64 operations each
-// where the compiler's division takes about 125 cycles).  LLE of 32^2 points 5.0 ->
-// 3.1 ms, a basin map of 231^2 points, one of them the fixed point at the origin,
-// 16.0 -> 5.9 ms, of 500^2 points 26.2 -> 23.7 ms.  The third divisor is known well
-// before its dividend, but its reciprocal taken ahead the same way made a step
-// longer (32^2 points: 3.7 ms): the compiler's reciprocal is a branch that nothing
-// overlaps.
+// where the compiler's division takes about 125 cycles).  Divisions as written against
+// these, the rest alike: LLE of 32^2 points (10 000 steps of a pair) 5.36 -> 4.23 ms,
+// of 500^2 27.9 -> 25.9 ms; basin maps of 231^2 points (50 000 steps), with the fixed
+// point at the origin on the grid 45.9 -> 18.7 ms, without it 18.8 -> 18.7, of 500^2
+// 78.2 ms both: a full SM hides the divisions' latency, one point's zeros hold up its
+// warp.  The third divisor is known well before its dividend, but its reciprocal taken
+// ahead the same way made a step a fifth longer: the compiler's reciprocal is a branch
+// that nothing overlaps.
 // A dividend out of range is divided as written, but for one that is no number, whose
 // quotient is none either: the spectra of 32^2 points without a bound, a third of which
 // leave the numbers, take 18.6 ms (24.1 with those divided too, 21.6 with the
