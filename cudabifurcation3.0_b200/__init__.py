@@ -390,10 +390,13 @@ def run_host(job: Job):
         else:
             cap = job.peakCapacity or L.cbf_record_length(C.byref(job))
         job.peakCapacity = cap
-        out = _peak_rows(n, cap) if job.task == TASK_PEAKS else np.zeros((n, cap), np.float64)
+        # the library's rows have one slot at least, also where there is nothing to record
+        out = _peak_rows(n, cap) if job.task == TASK_PEAKS else np.zeros((n, cap or 1), np.float64)
         aux = np.zeros(n, np.int32)
     check(L.cbf_run_host(C.byref(job), out.ctypes.data_as(C.c_void_p),
                          None if aux is None else aux.ctypes.data_as(C.c_void_p)))
+    if job.task == TASK_TRAJECTORY and cap == 0:
+        out = out[:, :0]
     return out, aux
 
 
