@@ -63,6 +63,7 @@ struct WarpArea {
 __device__ __forceinline__ void bif_epilogue(const BatchJob& B, long long p, int n, const BatchScratch& sc,
                                              long long slot, const WarpArea& wa, int lane, int* err)
 {
+    if (n < 0) return;  // done by its lane
     const double* pk = sc.peaks + slot * sc.stride;
     int r;
     if (B.job.task == CBF_TASK_KDE)
@@ -204,7 +205,17 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(
             {
                 const DevJob J = jobs[k].job;
                 n = go(J);
-                if (J.task != CBF_TASK_PEAKS) live = (int)min((long long)tilePts, J.nPoints - p0);
+                if (J.task != CBF_TASK_PEAKS) {
+                    // as in the maps: what the number of peaks decides is written at once
+                    int r = 0;
+                    const bool valid = lane < tilePts && p0 + lane < J.nPoints;
+                    if (valid)
+                        r = J.task == CBF_TASK_KDE ? kde_by_count(n, J.maxPeaks) : dbscan_by_count(n, J.maxPeaks);
+                    if (valid && r >= 0) ((int*)out)[p0 + lane] = r;
+                    const unsigned left = __ballot_sync(kFull, r < 0);
+                    if (r >= 0) n = -1;
+                    live = left ? highest_bit(left) + 1 : 0;
+                }
             }
             __syncwarp();
             epilogue_publish(sc.share, warpId, lane, n, live, t);
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(
         }
     }
     if constexpr (FAM == kFamPeaks)
-        epilogue_help(sc.share, warpId, lane, [&](long long from, unsigned long long t, int j) {
+        epilogue_help<4>(sc.share, warpId, lane, [&](long long from, unsigned long long t, int j) {
             long long p0 = 0;
             const int k = job_of(t, &p0);
             bif_epilogue(jobs[k], p0 + j, sc.share.count[from * 32 + j], sc, from * kTile + j, wa, lane, err);

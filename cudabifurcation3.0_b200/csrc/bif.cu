@@ -167,12 +167,19 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
         }
         __syncwarp();
 
-        const int live = (int)min((long long)tilePts, J.nPoints - tile * tilePts);
         if constexpr (task_shares(TASK)) {
-            epilogue_publish(sc.share, warpId, lane, over ? -1 : n, live, (unsigned long long)tile);
-            epilogue_own(sc.share, warpId, lane, live, [&](int j) { epilogue(warpId, tile, j); });
+            // what the number of peaks alone decides is written at once, and only the
+            // points up to the last of the others are published
+            int r = -1;
+            if (valid && !over) r = TASK == CBF_TASK_KDE ? kde_by_count(n, J.maxPeaks) : dbscan_by_count(n, J.maxPeaks);
+            if (r >= 0) ((int*)d_out)[p] = r;
+            const unsigned left = __ballot_sync(kFull, valid && !over && r < 0);
+            const int points = left ? highest_bit(left) + 1 : 0;
+            epilogue_publish(sc.share, warpId, lane, (left >> lane) & 1u ? n : -1, points, (unsigned long long)tile);
+            epilogue_own(sc.share, warpId, lane, points, [&](int j) { epilogue(warpId, tile, j); });
         } else {
             int res = 0;
+            const int live = (int)min((long long)tilePts, J.nPoints - tile * tilePts);
             for (int j = 0; j < live; ++j) {
                 const int nj = __shfl_sync(kFull, over ? 0 : n, j);
                 const int r = dbscan_warp(dbscan_spec(J), sc.peaks + (slot0 + j) * (long long)cap,
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(kBifThreads, kBifMinBlocks<S>) bif_kernel(cons
         }
     }
     if constexpr (task_shares(TASK))
-        epilogue_help(sc.share, warpId, lane,
+        epilogue_help<TASK == CBF_TASK_KDE ? 1 : 4>(sc.share, warpId, lane,
                       [&](long long from, unsigned long long tile, int j) { epilogue(from, (long long)tile, j); });
 }
 

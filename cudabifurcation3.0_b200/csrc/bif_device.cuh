@@ -423,6 +423,12 @@ __device__ __forceinline__ KdeSpec kde_spec(const DevJob& J)
     return KdeSpec{J.kdeI1, J.kdeI2, J.kdeH, J.kdeSkip, J.kdeInvH, J.maxPeaks, J.kdeSampling, J.kdeFixed};
 }
 
+// The count of a point that its number of peaks alone decides (-1: it does not).
+__device__ __forceinline__ int kde_by_count(int n, int maxPeaks)
+{
+    return n == 0 ? 0 : n <= 2 ? 1 : n > maxPeaks ? maxPeaks : -1;
+}
+
 // `keys`: room for keyCap floats of this warp, a power of two >= 32, 16-byte
 // aligned; in shared memory (SHARED) or in global memory.  A function of its own,
 // like the recorded loop: its registers are not the integration's.
@@ -430,9 +436,7 @@ template <bool SHARED>
 __device__ __noinline__ int kde_warp(const KdeSpec J, const double* pk, int n, int lane, float* keys, int keyCap)
 {
     float* key = SHARED ? static_cast<float*>(__cvta_shared_to_generic(__cvta_generic_to_shared(keys))) : keys;
-    if (n == 0) return 0;
-    if (n == 1 || n == 2) return 1;
-    if (n > J.maxPeaks) return J.maxPeaks;
+    if (n <= 2 || n > J.maxPeaks) return kde_by_count(n, J.maxPeaks);
 
     const double k1 = J.fixed ? (double)J.sampling : (double)(J.sampling * n);
     const double k2 = (J.i2 - J.i1) / (k1 - 1);
@@ -854,15 +858,19 @@ struct DbscanSpec {
 
 __device__ __forceinline__ DbscanSpec dbscan_spec(const DevJob& J) { return DbscanSpec{J.dbEps, J.dbSkip, J.maxPeaks}; }
 
+// The count of a point that its number of peaks alone decides (-1: it does not).
+__device__ __forceinline__ int dbscan_by_count(int n, int maxPeaks)
+{
+    return n <= 0 ? 0 : n == 1 ? 1 : n > maxPeaks ? 0 : -1;
+}
+
 // DBSCAN cluster count of one point; `so` (shared memory of this warp) enables
 // the sorted path for points with n - 1 <= so.cap peaks.
 __device__ __noinline__ int dbscan_warp(const DbscanSpec J, const double* pk,
                                         const double* iv, int n, int lane, unsigned* L,
                                         unsigned* Sb, int* err, DbscanSort so)
 {
-    if (n <= 0) return 0;
-    if (n == 1) return 1;
-    if (n > J.maxPeaks) return 0;
+    if (n <= 1 || n > J.maxPeaks) return dbscan_by_count(n, J.maxPeaks);
 
     const int words = (n + 31) >> 5;
     for (int w = lane; w < words; w += 32) {
@@ -959,11 +967,18 @@ __device__ __noinline__ int dbscan_warp(const DbscanSpec J, const double* pk,
 // the warps that find no tile left take other warps' points -- by an atomic
 // counter per warp.  A warp's peak slots are reused only with a new tile, which no
 // warp gets once others have found none: nothing a helper reads is overwritten.
+//
+// Taking a point is an atomic's round trip, so points that their number of peaks alone
+// decides are not shared: their lanes write them; and a look through all warps is a
+// round trip for every group of 32, so a helper looks only while a tile may have points.
+// Maps of next to no work (250^2 Lorenz points, 60 samples) take 62 us (DBSCAN) and 76
+// (KDE), 130 when every point was taken and every helper looked, 45 without sharing.
 struct EpilogueShare {
     unsigned* next;             // [warps] points taken of the published tile
     unsigned long long* info;   // [warps] published tile: payload << 6 | points
     int* count;                 // [warps * 32] emitted peaks of a point, -1: nothing to do
     unsigned* busy;             // warps that may hold a tile they have not published
+    unsigned* open;             // published tiles whose own warp has not taken their last point
     int warps;
 };
 
@@ -982,6 +997,7 @@ __host__ __device__ inline EpilogueShare epilogue_share(void* mem, long long war
     char* p = static_cast<char*>(mem);
     EpilogueShare sh;
     sh.busy = reinterpret_cast<unsigned*>(p);
+    sh.open = reinterpret_cast<unsigned*>(p + 128);
     sh.info = reinterpret_cast<unsigned long long*>(p + 256);
     sh.next = reinterpret_cast<unsigned*>(p + 256 + w * sizeof(unsigned long long));
     sh.count = reinterpret_cast<int*>(p + 256 + w * (sizeof(unsigned long long) + sizeof(unsigned)));
@@ -1003,14 +1019,20 @@ __device__ __forceinline__ unsigned long long epilogue_next_tile(const EpilogueS
     return __shfl_sync(kFull, t, 0);
 }
 
-// This warp's integrated tile: `n` per lane, `payload` names the tile.
+// This warp's integrated tile: `n` per lane, `payload` names the tile.  live = 0:
+// nothing is left to do, and what was published before has been taken.
 __device__ __forceinline__ void epilogue_publish(const EpilogueShare& sh, long long warp, int lane, int n, int live,
                                                  unsigned long long payload)
 {
+    if (live == 0) {
+        if (lane == 0) atomicSub(sh.busy, 1u);
+        return;
+    }
     sh.count[warp * 32 + lane] = n;
     __threadfence();  // peaks and counts before the tile
     __syncwarp();
     if (lane == 0) {
+        atomicAdd(sh.open, 1u);
         *(volatile unsigned long long*)(sh.info + warp) = payload << 6 | (unsigned)live;
         __threadfence();
         atomicExch(sh.next + warp, 0u);
@@ -1024,6 +1046,7 @@ __device__ __forceinline__ void epilogue_publish(const EpilogueShare& sh, long l
 template <class Item>
 __device__ __forceinline__ void epilogue_own(const EpilogueShare& sh, long long warp, int lane, int live, Item item)
 {
+    if (live == 0) return;
     unsigned j = 0;
     if (lane == 0) j = atomicAdd(sh.next + warp, 1u);
     j = __shfl_sync(kFull, j, 0);
@@ -1033,12 +1056,16 @@ __device__ __forceinline__ void epilogue_own(const EpilogueShare& sh, long long 
         item((int)j);
         j = __shfl_sync(kFull, after, 0);
     }
+    if (lane == 0) atomicSub(sh.open, 1u);
     __syncwarp();
 }
 
 // No tile is left: other warps' points until no warp holds a tile that it has not
 // published, or none has published one for kHelpIdle.  item(warp, payload, j).  A
-// helper that leaves early leaves the points to their own warp.
+// helper that leaves early leaves the points to their own warp.  LOOK: groups of 32
+// warps looked at at once -- four where a look is most of what helpers do (DBSCAN of
+// 496^2 Chen points 206 -> 186 ms, basin maps 2 to 4 % less), one beside the KDE
+// epilogue, whose registers are spilled for more (783^2 Rossler points 46 -> 48 ms).
 //
 // Why leave early: a waiting helper holds its place on the SM, and with it whatever
 // else is to run -- another stream's kernel, a batch's other family -- which matters
@@ -1055,43 +1082,77 @@ __device__ __forceinline__ unsigned long long now_ns()
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-template <class Item>
+template <int LOOK, class Item>
 __device__ __forceinline__ void epilogue_help(const EpilogueShare& sh, long long warp, int lane, Item item)
 {
     unsigned long long since = now_ns();
     for (int poll = 0; poll < kHelpPolls; ++poll) {
-        unsigned all = 0;
+        unsigned all = 0, none = 0;
         if (lane == 0) {
             all = *(volatile unsigned*)sh.busy == 0u;
             __threadfence();
+            none = all && *(volatile unsigned*)sh.open == 0u;  // as in a map of next to no work
         }
         all = __shfl_sync(kFull, all, 0);  // read before the look: nothing appears after it
+        if (__shfl_sync(kFull, none, 0)) return;
         bool found = false;
-        for (int base = 0; base < sh.warps; base += 32) {
-            // starts at the warp's own place, so that helpers spread
-            long long v = warp / 32 * 32 + base + lane;
-            if (v >= (sh.warps + 31) / 32 * 32) v -= (sh.warps + 31) / 32 * 32;
-            const bool some = v < sh.warps && *(volatile unsigned*)(sh.next + v) <
-                                                  (unsigned)(*(volatile unsigned long long*)(sh.info + v) & 63u);
-            unsigned mask = __ballot_sync(kFull, some);
-            while (mask) {
-                const int src = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const long long from = __shfl_sync(kFull, v, src);
-                for (;;) {
-                    unsigned j = 0;
-                    unsigned long long info = 0;
-                    if (lane == 0) {
-                        j = atomicAdd(sh.next + from, 1u);
-                        __threadfence();
-                        info = *(volatile unsigned long long*)(sh.info + from);
-                    }
-                    j = __shfl_sync(kFull, j, 0);
-                    info = __shfl_sync(kFull, info, 0);
-                    if (j >= (unsigned)(info & 63u)) break;
-                    __threadfence();  // the tile before its counts and peaks
-                    item(from, info >> 6, (int)j);
-                    found = true;
+        // warp `from`'s points, while there are any
+        auto take = [&](long long from) {
+            for (;;) {
+                unsigned j = 0;
+                unsigned long long info = 0;
+                if (lane == 0) {
+                    j = atomicAdd(sh.next + from, 1u);
+                    __threadfence();
+                    info = *(volatile unsigned long long*)(sh.info + from);
+                }
+                j = __shfl_sync(kFull, j, 0);
+                info = __shfl_sync(kFull, info, 0);
+                if (j >= (unsigned)(info & 63u)) break;
+                __threadfence();  // the tile before its counts and peaks
+                item(from, info >> 6, (int)j);
+                found = true;
+            }
+        };
+        // Both start at the warp's own group of 32, so that helpers spread.
+        if constexpr (LOOK == 1) {
+            for (int base = 0; base < sh.warps; base += 32) {
+                long long v = warp / 32 * 32 + base + lane;
+                if (v >= (sh.warps + 31) / 32 * 32) v -= (sh.warps + 31) / 32 * 32;
+                const bool some = v < sh.warps && *(volatile unsigned*)(sh.next + v) <
+                                                      (unsigned)(*(volatile unsigned long long*)(sh.info + v) & 63u);
+                unsigned mask = __ballot_sync(kFull, some);
+                while (mask) {
+                    const int src = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    take(__shfl_sync(kFull, v, src));
+                }
+            }
+        } else {
+            const int groups = (sh.warps + 31) / 32;
+            auto place = [&](int i) {
+                const int g = (int)(warp / 32) + i;
+                return g < groups ? g : g - groups;
+            };
+            for (int base = 0; base < groups; base += LOOK) {
+                unsigned next[LOOK], live[LOOK], masks[LOOK], any = 0;
+#pragma unroll
+                for (int k = 0; k < LOOK; ++k) {  // the loads together
+                    const int v = place(base + k) * 32 + lane;
+                    const bool there = base + k < groups && v < sh.warps;
+                    next[k] = there ? *(volatile unsigned*)(sh.next + v) : 0u;
+                    live[k] = there ? (unsigned)*(volatile unsigned long long*)(sh.info + v) & 63u : 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < LOOK; ++k) any |= masks[k] = __ballot_sync(kFull, next[k] < live[k]);
+                if (!any) continue;
+#pragma unroll 1
+                for (int k = 0; k < LOOK; ++k) {
+                    unsigned mask = masks[0];
+#pragma unroll
+                    for (int m = 1; m < LOOK; ++m)
+                        if (k == m) mask = masks[m];
+                    for (; mask; mask &= mask - 1) take(place(base + k) * 32ll + __ffs(mask) - 1);
                 }
             }
         }
@@ -1099,7 +1160,7 @@ __device__ __forceinline__ void epilogue_help(const EpilogueShare& sh, long long
             since = now_ns();
         } else {
             if (__shfl_sync(kFull, all || now_ns() - since > kHelpIdle, 0)) return;
-            __nanosleep(8000);
+            __nanosleep(8000);  // a map of little work ends at once
         }
     }
 }
