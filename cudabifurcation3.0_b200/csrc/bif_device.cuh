@@ -209,7 +209,8 @@ __device__ int integrate_point(const DevJob& J, long long g, double* pk, double*
         int t = 0;
         for (; t < J.nRecord; ++t) {
             traj[t] = phys_comp<S>(pick<D>(st.x, wv), wv, c);
-            for (int j = 0; j < J.preScaller; ++j) S::step(st.x, c);
+            for (int j = 0; j < J.preScaller - 1; ++j) S::step(st.x, c);
+            S::step(st.x, c);
             if (J.checkDiv && diverged(phys_comp<S>(pick<D>(st.x, wv), wv, c), J.divThresh)) {
                 div = true;
                 ++t;
