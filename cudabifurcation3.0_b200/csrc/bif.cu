@@ -209,11 +209,15 @@ __global__ void scatter_kernel(const T* __restrict__ src, const long long* __res
 // step, of which a warp issues 22), so it costs no more when fewer lanes of a
 // warp are in use, and the epilogues of a tile -- serial within a warp -- spread
 // over more warps (at four warps a step takes 90 cycles; with eight, 180).
-// (The 5-D model's step issues for half its latency: two warps per scheduler.)
+// The steps with a division issue for about half their latency: two warps per
+// scheduler for the 5-D model and Rossler (40^2 and 100^2 Rossler points, 9000 steps:
+// KDE 1.08 and 1.16 ms, with four 1.21 and 1.47; 40^2, 22 000 steps, peaks 2.07 and
+// 2.31, in tiles of 32 2.15).
 template <class S>
 int tile_points(long long n, int sms)
 {
-    const long long warps = (S::DIM == 3 ? 16ll : 8ll) * sms;
+    const bool divides = S::DIM == 5 || std::is_same<S, Rossler>::value;
+    const long long warps = (divides ? 8ll : 16ll) * sms;
     return (int)std::min(32ll, std::max(1ll, (n + warps - 1) / warps));
 }
 
