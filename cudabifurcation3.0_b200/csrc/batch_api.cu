@@ -252,7 +252,8 @@ cbf_status cbf_batch_create(const cbf_job* jobs, int32_t nJobs, void* const* d_o
     size_t share = 0;
     if (!b->fam[1].jobIdx.empty()) {
         // Tiles as in the peak maps (bif.cu: tile_points): 32 points, or fewer where
-        // that leaves less than four (with the 5-D model two) warps per scheduler.
+        // that leaves less than four (with the 5-D model two) warps per scheduler;
+        // Rossler jobs, usually some among others, do not change a batch's count.
         BatchFamily& F = b->fam[1];
         const long long warps = (F.withM5 ? 8ll : 16ll) * b->sms;
         F.tile = (int)std::min((long long)batch_tile(), std::max(1ll, (F.points + warps - 1) / warps));
